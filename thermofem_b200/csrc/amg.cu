@@ -232,6 +232,7 @@ class HierarchyImpl final : public Hierarchy {
     }
     ~HierarchyImpl() override {
         if (exec_) cudaGraphExecDestroy(exec_);
+        if (viewed_) wait_for_device();
     }
 
     void build(tf_ctx *ctx, const tf_dcsr &fine) {
@@ -539,6 +540,7 @@ class HierarchyImpl final : public Hierarchy {
     int level_count() const override { return static_cast<int>(levels_.size()); }
     tf_csr level_matrix(int d) const override {
         const auto &l = levels_.at(static_cast<size_t>(d));
+        viewed_ = true;
         const int vt = std::is_same_v<V, double> ? TF_F64 : TF_F32;
         tf_csr c{l.n, l.n, l.nnz, TF_I32, vt, l.rp.data(), l.ci.data(), l.val.data()};
         return c;
@@ -556,12 +558,14 @@ class HierarchyImpl final : public Hierarchy {
     void level_transfer(int d, const int32_t **map, const int32_t **off, const int32_t **mem,
                         int *coarse) const override {
         const auto &l = levels_.at(static_cast<size_t>(d));
+        viewed_ = true;
         *map = l.map.data();
         *off = l.off.data();
         *mem = l.mem.data();
         *coarse = l.coarse;
     }
     void coarse_factor(int *rows, const double **lu, const int32_t **pivots) const override {
+        viewed_ = true;
         *rows = factored_ ? static_cast<int>(levels_.back().n) : 0;
         *lu = factored_ ? lu_.data() : nullptr;
         *pivots = factored_ ? piv_.data() : nullptr;
@@ -1092,6 +1096,9 @@ class HierarchyImpl final : public Hierarchy {
     DeviceBuffer<double> lu_, inv_;
     DeviceBuffer<int32_t> piv_;
     bool factored_{false};
+    // a caller was given device pointers into the hierarchy, which it may be
+    // reading on streams of its own
+    mutable bool viewed_{false};
     cudaGraphExec_t exec_{nullptr};
     bool capture_failed_{false};
     int64_t per_cycle_{0};

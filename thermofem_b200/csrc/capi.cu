@@ -137,6 +137,9 @@ int tf_ctx_create(int device, void *stream, tf_ctx **out) {
             cuda_check(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "cudaStreamCreate");
             ctx->own_stream = true;
         }
+        auto life = std::make_shared<StreamLife>(StreamLife{ctx->stream, device, true});
+        pool_context_opened(device);
+        ctx->life = std::move(life);
         cuda_check(cudaMallocHost(&ctx->pinned, 256), "cudaMallocHost");
         cuda_check(cudaMalloc(&ctx->fault, sizeof(int)), "cudaMalloc");
         cuda_check(cudaMemsetAsync(ctx->fault, 0, sizeof(int), ctx->stream), "cudaMemsetAsync");
@@ -215,6 +218,7 @@ int tf_canonicalize(tf_ctx *ctx, const tf_csr *a, tf_dcsr **out) {
         require(c.rows > 0 && c.rows < INT32_MAX && c.nnz <= INT32_MAX / 2,
                 "AMG requires nonempty square int32-capacity CSR on workspace device");
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         const int flags = csr_canonical_flags(ctx, c);
         if (flags & 2) fail(TF_ERR_INVALID, "AMG invalid CSR or nonfinite coefficient");
         if (flags == 0) {
@@ -546,6 +550,7 @@ int tf_strength(tf_ctx *ctx, const tf_csr *a, const double *row_max, double thre
         auto c = native_csr(a);
         require(c.rows > 0, "empty matrix");
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         auto g = strength_graph(ctx, c, row_max, threshold);
         cuda_check(cudaStreamSynchronize(ctx->stream), "strength");
         *graph = g.release();
@@ -559,6 +564,7 @@ int tf_match(tf_ctx *ctx, const tf_csr *graph, int rounds, int32_t *map, int *co
         auto g = native_csr(graph);
         require(g.rows > 0, "empty graph");
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         *count = match_pairs(ctx, g, rounds, map);
     });
 }
@@ -570,6 +576,7 @@ int tf_contract(tf_ctx *ctx, const tf_csr *graph, const int32_t *map, int count,
         *out = nullptr;
         auto g = native_csr(graph);
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         auto c = contract_graph(ctx, g, map, count);
         cuda_check(cudaStreamSynchronize(ctx->stream), "contract");
         *out = c.release();
@@ -584,6 +591,7 @@ int tf_aggregate(tf_ctx *ctx, const tf_csr *graph, int rounds, int absorb_single
         require(rounds >= 1 && rounds <= 8 && graph && graph->rows > 0, "Invalid matching configuration");
         auto g = native_csr(graph);
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         *out = aggregate(ctx, g, rounds, absorb_singletons != 0).release();
     });
 }
@@ -619,6 +627,7 @@ int tf_galerkin(tf_ctx *ctx, const tf_csr *a, const tf_transfer *t, tf_dcsr **ou
         auto c = native_csr(a);
         require(c.rows == t->fine_rows && t->coarse_rows >= 1, "AMG transfer dimension mismatch");
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         auto m = galerkin(ctx, c, t->map.data(), t->coarse_rows);
         cuda_check(cudaStreamSynchronize(ctx->stream), "galerkin");
         *out = m.release();
@@ -633,6 +642,7 @@ int tf_galerkin_map(tf_ctx *ctx, const tf_csr *a, const int32_t *map, int coarse
         auto c = native_csr(a);
         require(coarse_rows >= 1 && coarse_rows <= c.rows, "AMG transfer dimension mismatch");
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         if (indices_out_of_range(ctx, c.rows, map, coarse_rows))
             fail(TF_ERR_INVALID, "aggregate map entry outside 0..coarse_rows-1");
         auto m = galerkin(ctx, c, map, coarse_rows);
@@ -648,6 +658,7 @@ int tf_radix_sort_pairs_u64f64(tf_ctx *ctx, int64_t n, const uint64_t *keys_in, 
         require_vectors(n, {keys_in, values_in, keys_out, values_out}, "invalid sort arguments");
         require(n == 0 || (keys_in != keys_out && values_in != values_out), "sort outputs must not alias inputs");
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         radix_sort_pairs(ctx, n, keys_in, values_in, keys_out, values_out, end_bit);
     });
 }
@@ -659,6 +670,7 @@ int tf_reduce_by_key_u64f64(tf_ctx *ctx, int64_t n, const uint64_t *keys, const 
         require(count != nullptr && (op == 0 || op == 1), "invalid reduce arguments");
         require_vectors(n, {keys, values, keys_out, values_out}, "invalid reduce arguments");
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         *count = reduce_by_key(ctx, n, keys, values, op, keys_out, values_out);
     });
 }
@@ -668,6 +680,7 @@ int tf_scan_exclusive_i32(tf_ctx *ctx, int64_t n, const int32_t *in, int32_t *ou
         check_ctx(ctx);
         require_vectors(n, {in, out}, "invalid scan arguments");
         DeviceScope scope(ctx->device);
+        PoolTrim trim(ctx);
         scan_exclusive(ctx, n, in, out);
     });
 }

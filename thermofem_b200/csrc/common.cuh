@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <stdexcept>
 #include <string>
@@ -80,8 +81,35 @@ class DeviceScope {
     int previous_{0};
 };
 
-// Owning device allocation (cudaMalloc / cudaFree).  Allocation happens in
-// setup and workspace growth only; the solve loop never allocates.
+// A context's stream, shared with the pool buffers allocated on it: while
+// open, a buffer is freed in the stream's order; once the context is
+// destroyed (its stream has drained then), directly.
+struct StreamLife {
+    cudaStream_t stream{nullptr};
+    int device{0};
+    bool open{true};
+};
+
+// The device memory pool (pool.cu): allocation in stream order; free bytes
+// beyond a bound go back to the device at pool_trim().
+void *pool_allocate(int device, cudaStream_t stream, size_t bytes);
+void pool_trim(int device) noexcept;
+void pool_context_opened(int device);
+void pool_context_closed(int device) noexcept;
+// Waits for all work queued on the current device, on whatever stream, as
+// cudaFree does (cudaDeviceSynchronize would break another thread's stream
+// capture).
+void wait_for_device() noexcept;
+
+// The stream on which this thread's DeviceBuffers are allocated from the
+// pool, null outside PoolScope.
+inline thread_local const std::shared_ptr<StreamLife> *pool_stream = nullptr;
+
+// Owning device allocation.  Inside a PoolScope (component setups) it comes
+// from the device's pool and is used and freed in the order of the context's
+// stream; elsewhere (what a caller may hold or read on streams of its own)
+// it is a cudaMalloc, whose cudaFree waits for the device.  Allocation
+// happens in setup and workspace growth only; the solve loop never allocates.
 template <class T>
 class DeviceBuffer {
   public:
@@ -102,10 +130,15 @@ class DeviceBuffer {
         std::swap(ptr_, o.ptr_);
         std::swap(size_, o.size_);
         std::swap(device_, o.device_);
+        std::swap(life_, o.life_);
     }
     void allocate(size_t n) {
         release();
-        if (n) {
+        if (n && pool_stream) {
+            ptr_ = pool_allocate((*pool_stream)->device, (*pool_stream)->stream, n * sizeof(T));
+            life_ = *pool_stream;
+            device_ = life_->device;
+        } else if (n) {
             cuda_check(cudaGetDevice(&device_), "cudaGetDevice");
             cuda_check(cudaMalloc(&ptr_, n * sizeof(T)), "cudaMalloc");
         }
@@ -120,9 +153,15 @@ class DeviceBuffer {
             int now = -1;
             cudaGetDevice(&now);
             if (now != device_) cudaSetDevice(device_);
-            cudaFree(ptr_);
+            if (life_ && life_->open) {
+                cudaFreeAsync(ptr_, life_->stream);
+            } else {
+                cudaFree(ptr_);
+                if (life_) pool_trim(device_);
+            }
             if (now != device_) cudaSetDevice(now);
         }
+        life_.reset();
         ptr_ = nullptr;
         size_ = 0;
     }
@@ -134,6 +173,7 @@ class DeviceBuffer {
     void *ptr_{nullptr};
     size_t size_{0};
     int device_{-1};
+    std::shared_ptr<StreamLife> life_;  // of a pool buffer
 };
 
 }  // namespace tfb
@@ -153,6 +193,7 @@ struct tf_ctx {
     bool pdl{true};                             // launch_kernel adds programmatic dependent launch
     bool stable{false};                         // operators are read-only (solve / cycle enqueue)
     bool checked{false};                        // caller CSR validated before kernel-layer launches
+    std::shared_ptr<tfb::StreamLife> life;      // of pool buffers on this context's stream
     tf_ctx() = default;
     tf_ctx(const tf_ctx &) = delete;
     tf_ctx &operator=(const tf_ctx &) = delete;
@@ -160,6 +201,10 @@ struct tf_ctx {
     // (the caller makes the context's device current).
     ~tf_ctx() {
         if (stream) cudaStreamSynchronize(stream);
+        if (life) {
+            life->open = false;
+            tfb::pool_context_closed(device);
+        }
         scratch.release();
         scratch2.release();
         if (pinned) cudaFreeHost(pinned);
@@ -177,6 +222,55 @@ struct tf_ctx {
 namespace tfb {
 
 constexpr int kBlock = 256;
+
+// DeviceBuffers of this thread come from the pool, on ctx's stream, while
+// the scope lives; at its end the pool gives back what exceeds its bound.
+class PoolScope {
+  public:
+    explicit PoolScope(const tf_ctx *ctx) : previous_(pool_stream), device_(ctx->device) { pool_stream = &ctx->life; }
+    ~PoolScope() {
+        pool_stream = previous_;
+        pool_trim(device_);
+    }
+    PoolScope(const PoolScope &) = delete;
+    PoolScope &operator=(const PoolScope &) = delete;
+
+  private:
+    const std::shared_ptr<StreamLife> *previous_;
+    int device_;
+};
+
+// Ends a call that used temporary arrays: the pool gives back what exceeds
+// its bound.
+struct PoolTrim {
+    int device;
+    explicit PoolTrim(const tf_ctx *ctx) : device(ctx->device) {}
+    ~PoolTrim() { pool_trim(device); }
+    PoolTrim(const PoolTrim &) = delete;
+    PoolTrim &operator=(const PoolTrim &) = delete;
+};
+
+// Temporary device array, allocated and freed in the order of the context's
+// stream.
+template <class T>
+class TempBuffer {
+  public:
+    TempBuffer(tf_ctx *ctx, size_t n) : ctx_(ctx), n_(n) {
+        if (n) p_ = pool_allocate(ctx->device, ctx->stream, n * sizeof(T));
+    }
+    ~TempBuffer() {
+        if (p_) cudaFreeAsync(p_, ctx_->stream);
+    }
+    TempBuffer(const TempBuffer &) = delete;
+    TempBuffer &operator=(const TempBuffer &) = delete;
+    T *data() const { return static_cast<T *>(p_); }
+    size_t size() const { return n_; }
+
+  private:
+    tf_ctx *ctx_;
+    size_t n_;
+    void *p_{nullptr};
+};
 
 inline unsigned grid_for(int64_t n, int block = kBlock) {
     int64_t g = (n + block - 1) / block;

@@ -58,6 +58,13 @@ void check_types(int value_type, int index_type) {
     require(index_type == TF_I32 || index_type == TF_I64, "index type must be TF_I32 or TF_I64");
 }
 
+// After a component's buffers were freed (in the order of the context's
+// stream): they are the pool's once the stream has drained.
+void released(tf_ctx *ctx) {
+    cudaStreamSynchronize(ctx->stream);
+    pool_trim(ctx->device);
+}
+
 void check_matrix_types(const tf_csr *a, int value_type, int index_type) {
     check_csr(a);
     require(a->value_type == value_type && a->index_type == index_type, "matrix types differ from the component's");
@@ -107,8 +114,10 @@ int tf_amg_create(tf_ctx *ctx, int value_type, int index_type, const tf_amg_opti
 int tf_amg_destroy(tf_amg *m) {
     return guard([&] {
         if (!m) return;
-        DeviceScope scope(m->ctx->device);
+        tf_ctx *ctx = m->ctx;
+        DeviceScope scope(ctx->device);
         delete m;
+        released(ctx);
     });
 }
 
@@ -118,6 +127,7 @@ int tf_amg_setup(tf_amg *m, const tf_csr *a) {
         check_matrix_types(a, m->value_type, m->index_type);
         require(a->rows > 0 && a->rows == a->cols, "Solver requires a nonempty square matrix");
         DeviceScope scope(m->ctx->device);
+        PoolScope pool(m->ctx);
         auto native = to_native(m->ctx, *a);
         const int storage = m->cfg.o.hierarchy_type == -1 ? m->value_type : m->cfg.o.hierarchy_type;
         auto h = build_hierarchy(m->ctx, m->cfg, storage, *native);
@@ -249,6 +259,7 @@ int tf_amg_load(tf_amg *m, const char *path) {
         if (!in) fail(TF_ERR_INVALID, std::string("AMG checkpoint: cannot open ") + path);
         const int storage = m->cfg.o.hierarchy_type == -1 ? m->value_type : m->cfg.o.hierarchy_type;
         // transactional, as setup: the previous hierarchy stays on failure
+        PoolScope pool(m->ctx);
         auto h = restore_hierarchy(m->ctx, m->cfg, storage, in);
         m->owned = std::move(h);
         m->h = m->owned.get();
@@ -276,8 +287,10 @@ int tf_jacobi_create(tf_ctx *ctx, int value_type, int index_type, int sweeps, do
 int tf_jacobi_destroy(tf_jacobi *j) {
     return guard([&] {
         if (!j) return;
-        DeviceScope scope(j->ctx->device);
+        tf_ctx *ctx = j->ctx;
+        DeviceScope scope(ctx->device);
         delete j;
+        released(ctx);
     });
 }
 
@@ -288,6 +301,7 @@ int tf_jacobi_setup(tf_jacobi *j, const tf_csr *a) {
         require(a->rows > 0 && a->rows == a->cols, "Solver requires a nonempty square matrix");
         DeviceScope scope(j->ctx->device);
         tf_ctx *ctx = j->ctx;
+        PoolScope pool(ctx);
         std::unique_ptr<tf_dcsr> native;
         try {
             native = to_native(ctx, *a);
@@ -374,8 +388,10 @@ int tf_solver_create(tf_ctx *ctx, int kind, int value_type, int index_type, cons
 int tf_solver_destroy(tf_solver *s) {
     return guard([&] {
         if (!s) return;
-        DeviceScope scope(s->ctx->device);
+        tf_ctx *ctx = s->ctx;
+        DeviceScope scope(ctx->device);
         delete s;
+        released(ctx);
     });
 }
 
@@ -384,6 +400,7 @@ int tf_solver_setup(tf_solver *s, const tf_csr *a) {
         require(s != nullptr, "null solver");
         check_matrix_types(a, s->value_type, s->index_type);
         DeviceScope scope(s->ctx->device);
+        PoolScope pool(s->ctx);
         s->view.reset();
         s->k->setup(s->ctx, *a);
     });

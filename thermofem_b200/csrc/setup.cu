@@ -15,26 +15,8 @@
 namespace tfb {
 namespace {
 
-// Stream-ordered temporary allocation (cudaMallocAsync / cudaFreeAsync).
 template <class T>
-class Temp {
-  public:
-    Temp(tf_ctx *ctx, size_t n) : ctx_(ctx), n_(n) {
-        if (n) cuda_check(cudaMallocAsync(&p_, n * sizeof(T), ctx->stream), "cudaMallocAsync");
-    }
-    ~Temp() {
-        if (p_) cudaFreeAsync(p_, ctx_->stream);
-    }
-    Temp(const Temp &) = delete;
-    Temp &operator=(const Temp &) = delete;
-    T *data() const { return static_cast<T *>(p_); }
-    size_t size() const { return n_; }
-
-  private:
-    tf_ctx *ctx_;
-    size_t n_;
-    void *p_{nullptr};
-};
+using Temp = TempBuffer<T>;
 
 __device__ __forceinline__ uint64_t sort_key(int r, int c, int bits) {
     return (static_cast<uint64_t>(static_cast<unsigned>(r)) << bits) | static_cast<unsigned>(c);

@@ -21,25 +21,6 @@ constexpr int kSortRounds = 16;
 constexpr int kSortTile = kSortThreads * kSortRounds;
 constexpr int kDigits = 256;
 
-// Stream-ordered temporary allocation (cudaMallocAsync / cudaFreeAsync).
-template <class T>
-class TempBuffer {
-  public:
-    TempBuffer(tf_ctx *ctx, size_t n) : ctx_(ctx) {
-        if (n) cuda_check(cudaMallocAsync(&p_, n * sizeof(T), ctx->stream), "cudaMallocAsync");
-    }
-    ~TempBuffer() {
-        if (p_) cudaFreeAsync(p_, ctx_->stream);
-    }
-    TempBuffer(const TempBuffer &) = delete;
-    TempBuffer &operator=(const TempBuffer &) = delete;
-    T *data() const { return static_cast<T *>(p_); }
-
-  private:
-    tf_ctx *ctx_;
-    void *p_{nullptr};
-};
-
 // Block-wide exclusive scan of kScanItems consecutive items per thread.
 // Returns the block total; out[k] = exclusive prefix of item k of this thread.
 __device__ __forceinline__ int block_scan(int (&v)[kScanItems], int *warp_tot) {
