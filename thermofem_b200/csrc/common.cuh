@@ -201,12 +201,13 @@ struct tf_ctx {
     // (the caller makes the context's device current).
     ~tf_ctx() {
         if (stream) cudaStreamSynchronize(stream);
+        scratch.release();
+        scratch2.release();
         if (life) {
+            if (stream) cudaStreamSynchronize(stream);  // the arenas' frees
             life->open = false;
             tfb::pool_context_closed(device);
         }
-        scratch.release();
-        scratch2.release();
         if (pinned) cudaFreeHost(pinned);
         if (fault) cudaFree(fault);
         if (own_stream && stream) cudaStreamDestroy(stream);
