@@ -23,6 +23,7 @@
 #include "coarse_cycle.cuh"
 #include "engine.cuh"
 #include "mlp.cuh"
+#include "setup.cuh"
 
 namespace tfb {
 
@@ -294,7 +295,7 @@ class HierarchyImpl final : public Hierarchy {
                 break;
             }
             marks.mark(ctx, kPhGalerkin);
-            auto coarse = galerkin(ctx, nc, t->map.data(), t->coarse_rows);
+            auto coarse = galerkin(ctx, nc, *t);
             for (int k = 0; k < 4; ++k) stats.back().histogram[k] = t->histogram[k];
             l.map = std::move(t->map);
             l.off = std::move(t->offsets);

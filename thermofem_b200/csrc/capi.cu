@@ -1,7 +1,7 @@
 // capi.cu -- extern "C" entry points of the kernel layer (thermofem_b200.h).
 // Each validates its POD arguments, dispatches on element types and calls
 // the typed entry points of ops.cuh on the context's stream.
-#include "ops.cuh"
+#include "setup.cuh"
 
 #include <cstdio>
 #include <cstdlib>
@@ -628,7 +628,7 @@ int tf_galerkin(tf_ctx *ctx, const tf_csr *a, const tf_transfer *t, tf_dcsr **ou
         require(c.rows == t->fine_rows && t->coarse_rows >= 1, "AMG transfer dimension mismatch");
         DeviceScope scope(ctx->device);
         PoolTrim trim(ctx);
-        auto m = galerkin(ctx, c, t->map.data(), t->coarse_rows);
+        auto m = galerkin(ctx, c, *t);
         cuda_check(cudaStreamSynchronize(ctx->stream), "galerkin");
         *out = m.release();
     });

@@ -210,24 +210,8 @@ int csr_canonical_flags(tf_ctx *ctx, const Csr<T, I> &a);
 // Finite values, nonfinite entry or bad diagonal -> false; row max |offdiag|.
 bool row_stats(tf_ctx *ctx, const Csr<double, int32_t> &a, double *row_max);
 
-// Sorting primitives (sort.cu).
-void radix_sort_pairs(tf_ctx *ctx, int64_t n, const uint64_t *kin, const double *vin, uint64_t *kout,
-                      double *vout, int end_bit);
-int64_t reduce_by_key(tf_ctx *ctx, int64_t n, const uint64_t *keys, const double *vals, int op, uint64_t *kout,
-                      double *vout);
+// Exclusive scan (sort.cu).
 void scan_exclusive(tf_ctx *ctx, int64_t n, const int32_t *in, int32_t *out);
-
-// Coordinate compression (sort + reduce + unpack) into an owned CSR.
-std::unique_ptr<tf_dcsr> compress(tf_ctx *ctx, int rows, int64_t n, const uint64_t *keys, const double *vals, int col_bits, int op);
-int column_bits(int rows);
-
-// Setup stages (setup.cu), on canonical FP64/int32 operands.
-std::unique_ptr<tf_dcsr> canonicalize(tf_ctx *ctx, const Csr<double, int32_t> &a);
-std::unique_ptr<tf_dcsr> strength_graph(tf_ctx *ctx, const Csr<double, int32_t> &a, const double *row_max, double theta);
-int match_pairs(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, int32_t *map);
-std::unique_ptr<tf_dcsr> contract_graph(tf_ctx *ctx, const Csr<double, int32_t> &g, const int32_t *map, int count);
-std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, bool absorb);
-std::unique_ptr<tf_dcsr> galerkin(tf_ctx *ctx, const Csr<double, int32_t> &a, const int32_t *map, int coarse);
 
 // Coarse LU (coarse.cu).
 bool coarse_lu_factor(tf_ctx *ctx, const Csr<double, int32_t> &a, double *lu, int32_t *pivots);

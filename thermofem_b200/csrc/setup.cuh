@@ -1,0 +1,29 @@
+// setup.cuh -- typed entry points of the sorting primitives (sort.cu) and of
+// the aggregation setup's stages (setup.cu).
+#pragma once
+#include "ops.cuh"
+
+namespace tfb {
+
+// Sorting primitives (sort.cu).
+void radix_sort_pairs(tf_ctx *ctx, int64_t n, const uint64_t *kin, const double *vin, uint64_t *kout,
+                      double *vout, int end_bit);
+int64_t reduce_by_key(tf_ctx *ctx, int64_t n, const uint64_t *keys, const double *vals, int op, uint64_t *kout,
+                      double *vout);
+
+// Coordinate compression (sort + reduce + unpack) into an owned CSR.
+std::unique_ptr<tf_dcsr> compress(tf_ctx *ctx, int rows, int64_t n, const uint64_t *keys, const double *vals, int col_bits, int op);
+int column_bits(int rows);
+
+// Setup stages (setup.cu), on canonical FP64/int32 operands.
+std::unique_ptr<tf_dcsr> canonicalize(tf_ctx *ctx, const Csr<double, int32_t> &a);
+std::unique_ptr<tf_dcsr> strength_graph(tf_ctx *ctx, const Csr<double, int32_t> &a, const double *row_max, double theta);
+int match_pairs(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, int32_t *map);
+std::unique_ptr<tf_dcsr> contract_graph(tf_ctx *ctx, const Csr<double, int32_t> &g, const int32_t *map, int count);
+std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, bool absorb);
+// P^T A P for any map, by a sort over all coordinates, and for a transfer's
+// aggregates (at most four members), row by row; the same bits.
+std::unique_ptr<tf_dcsr> galerkin(tf_ctx *ctx, const Csr<double, int32_t> &a, const int32_t *map, int coarse);
+std::unique_ptr<tf_dcsr> galerkin(tf_ctx *ctx, const Csr<double, int32_t> &a, const tf_transfer &t);
+
+}  // namespace tfb

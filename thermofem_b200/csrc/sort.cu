@@ -7,7 +7,7 @@
 // one thread from left to right, so Galerkin and canonical sums come out in
 // the order the reference's host oracle uses (stable sort, then sequential
 // sum), independent of the GPU.
-#include "ops.cuh"
+#include "setup.cuh"
 
 namespace tfb {
 namespace {
