@@ -10,6 +10,9 @@
 // any are accepted, absorption reads the pre-round map and sizes, member
 // slots are re-sorted after the atomic fill.  Sorting, reduction and scans
 // are the project's own (sort.cu).
+#include <climits>
+
+#include "scan.cuh"
 #include "setup.cuh"
 
 namespace tfb {
@@ -72,55 +75,151 @@ __global__ void strength_edges(int n, const int32_t *__restrict__ rp, const int3
     if (!keys) count[i] = pos;
 }
 
-// Each unmatched vertex proposes its best unmatched neighbour from one
-// snapshot of mate[] (GpuAggregation.cu:402-431).
-__global__ void propose(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
-                        const double *__restrict__ w, const int32_t *__restrict__ mate, int32_t *__restrict__ proposal) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// The vertices of a matching: the rows themselves, or pairs of rows (lo, hi;
+// hi < 0 for a single row) with map giving the pair of every row.  The graph
+// over pairs is never formed: a pair's edges are its rows' edges seen through
+// map, and a proposal (the best edge to an unmatched vertex) comes out the
+// same whether parallel edges are merged by their maximum first or not.
+struct Vertices {
+    const int32_t *lo{nullptr}, *hi{nullptr}, *map{nullptr};
+    const int32_t *count{nullptr};  // their number, when the host does not know it
+    int n{0};                       // their number, or a bound of it
+    __device__ __forceinline__ int size() const { return count ? *count : n; }
+    __device__ __forceinline__ int of(int row) const { return map ? map[row] : row; }
+};
+
+// State of a matching between rounds: mate[] (-1 unmatched) as of the
+// proposals before last, and the last round's proposals, not yet accepted:
+// a mutual pair among them is matched.  Vertex v's own thread writes that
+// into mate[v] in the next round; readers that still find -1 there come to
+// the same answer from the proposals.
+__device__ __forceinline__ int mate_of(int v, const int32_t *mate, const int32_t *last) {
+    const int m = mate[v];
+    if (m >= 0 || !last) return m;
+    const int p = last[v];
+    return p >= 0 && last[p] == v ? p : -1;
+}
+
+// (s, c) beats (score, best) as v's proposal (GpuAggregation.cu:402-431):
+// larger weight, then larger edge priority, then smaller vertex.
+__device__ __forceinline__ bool better(int v, double s, int c, double score, int best) {
+    if (s != score) return s > score;
+    if (c < 0 || c == best) return false;
+    if (best < 0) return s > 0;
+    const uint64_t a = edge_priority(v, c), b = edge_priority(v, best);
+    return a > b || (a == b && c < best);
+}
+
+// One handshake round: accepts the last round's mutual proposals
+// (GpuAggregation.cu:440-449) and writes this round's: each unmatched vertex
+// proposes its best unmatched neighbour, from one snapshot of the matching.
+// kG lanes share a vertex.
+//
+// Bound: the gathers of the neighbours' state.  Acceptance in the next
+// round's kernel halves the launches of a matching; weights are read first,
+// and only an edge that would win gathers its neighbour.
+template <int kG>
+__global__ void match_round(Vertices vs, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                            const double *__restrict__ w, int32_t *mate, const int32_t *__restrict__ last,
+                            int32_t *__restrict__ proposal) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const int lane = static_cast<int>(t % kG);
+    const int nv = vs.size();
+    if (t / kG >= nv) return;  // uniform over the vertex's lanes
+    const int v = static_cast<int>(t / kG);
+    const int mine = mate_of(v, mate, last);
+    if (mine >= 0) {
+        if (lane == 0) {
+            mate[v] = mine;
+            proposal[v] = -1;
+        }
+        return;
+    }
     int best = -1;
     double score = 0;
-    uint64_t priority = 0;
-    if (mate[i] < 0) {
-        for (int32_t j = rp[i]; j < rp[i + 1]; ++j) {
-            const int c = ci[j];
+    for (int k = 0; k < 2; ++k) {
+        const int row = vs.lo ? (k ? vs.hi[v] : vs.lo[v]) : (k ? -1 : v);
+        if (row < 0) break;
+        for (int32_t j = rp[row] + lane; j < rp[row + 1]; j += kG) {
             const double s = w[j];
-            if (c == i || mate[c] >= 0 || s <= 0 || s < score) continue;
-            const uint64_t cand = edge_priority(i, c);
-            if (s > score || (s == score && (best < 0 || cand > priority || (cand == priority && c < best)))) {
+            if (!(s > 0) || s < score) continue;
+            const int c = vs.of(ci[j]);
+            if (c == v || !better(v, s, c, score, best) || mate_of(c, mate, last) >= 0) continue;
+            best = c;
+            score = s;
+        }
+    }
+    if constexpr (kG > 1) {
+        const unsigned group = (kG == 32 ? 0xffffffffu : ((1u << (kG & 31)) - 1u))
+                               << ((threadIdx.x & 31) / kG * kG);
+#pragma unroll
+        for (int o = kG / 2; o > 0; o >>= 1) {
+            const double s = __shfl_xor_sync(group, score, o);
+            const int c = __shfl_xor_sync(group, best, o);
+            if (better(v, s, c, score, best)) {
                 best = c;
                 score = s;
-                priority = cand;
             }
         }
     }
-    proposal[i] = best;
+    if (lane == 0) proposal[v] = best;
 }
 
-// Mutual proposals become pairs (GpuAggregation.cu:440-449).
-__global__ void accept(int n, const int32_t *__restrict__ proposal, int32_t *__restrict__ mate) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int p = proposal[i];
-    if (p >= 0 && proposal[p] == i) mate[i] = p;
-}
+// Scan input: 1 for the vertex that stands for its pair (or itself alone).
+struct RootFlag {
+    Vertices vs;
+    const int32_t *mate, *last;
+    __device__ Counts<1> operator()(int v) const {
+        if (v >= vs.size()) return {0};
+        const int m = mate_of(v, mate, last);
+        return {m < 0 || v < m ? 1 : 0};
+    }
+};
 
-// Root flags with a zero sentinel at n (GpuAggregation.cu:458-463).
-__global__ void roots(int n, const int32_t *__restrict__ mate, int32_t *__restrict__ flags) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= n) flags[i] = (i < n && (mate[i] < 0 || i < mate[i])) ? 1 : 0;
-}
+// Scan output over the rows' matching: pair k = (lo, hi), map of its rows;
+// position n carries the number of pairs.
+struct AssignPairs {
+    RootFlag f;
+    int32_t *lo, *hi, *map, *count;
+    __device__ void operator()(int v, const Counts<1> &flag, const Counts<1> &before) const {
+        const int k = before.v[0];
+        if (v == f.vs.n) *count = k;
+        if (!flag.v[0]) return;
+        const int m = mate_of(v, f.mate, f.last);
+        if (lo) {
+            lo[k] = v;
+            hi[k] = m;
+        }
+        map[v] = k;
+        if (m >= 0) map[m] = k;
+    }
+};
 
-__global__ void assign(int n, const int32_t *__restrict__ mate, const int32_t *__restrict__ prefix,
-                       int32_t *__restrict__ map) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) map[i] = prefix[mate[i] < 0 ? i : min(i, mate[i])];
-}
-
-__global__ void compose(int n, int32_t *__restrict__ map, const int32_t *__restrict__ second) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) map[i] = second[map[i]];
-}
+// Scan output over the pairs' matching: the rows of aggregate k (at most
+// four), its size and the map of its rows.
+struct AssignAggregates {
+    RootFlag f;
+    int32_t *slots, *sizes, *map, *count;
+    __device__ void operator()(int v, const Counts<1> &flag, const Counts<1> &before) const {
+        const int k = before.v[0];
+        if (v == f.vs.n) *count = k;
+        if (!flag.v[0]) return;
+        int size = 0;
+        auto add = [&](int row) {
+            if (row < 0) return;
+            slots[static_cast<int64_t>(k) * 4 + size++] = row;
+            map[row] = k;
+        };
+        const int m = mate_of(v, f.mate, f.last);
+        add(f.vs.lo[v]);
+        add(f.vs.hi[v]);
+        if (m >= 0) {
+            add(f.vs.lo[m]);
+            add(f.vs.hi[m]);
+        }
+        sizes[k] = size;
+    }
+};
 
 // Cross-aggregate edges of the graph under map (GpuAggregation.cu:534-553).
 __global__ void map_graph(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
@@ -141,34 +240,6 @@ __global__ void map_graph(int n, const int32_t *__restrict__ rp, const int32_t *
         }
     }
     if (!keys) offsets[i] = pos;
-}
-
-// Four-slot member table filled by integer atomics (GpuAggregation.cu:586-593);
-// the slot order is then fixed by sort_members.
-__global__ void slot_members(int n, const int32_t *__restrict__ map, int32_t *__restrict__ sizes,
-                             int32_t *__restrict__ slots, int *overflow) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int c = map[i];
-    const int slot = atomicAdd(sizes + c, 1);
-    if (slot < 4) slots[static_cast<int64_t>(c) * 4 + slot] = i;
-    else atomicExch(overflow, 1);
-}
-
-__global__ void sort_members(int n, const int32_t *__restrict__ sizes, int32_t *__restrict__ slots) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    int32_t *m = slots + static_cast<int64_t>(c) * 4;
-    const int s = min(sizes[c], 4);
-    for (int i = 1; i < s; ++i) {
-        const int v = m[i];
-        int j = i;
-        while (j > 0 && m[j - 1] > v) {
-            m[j] = m[j - 1];
-            --j;
-        }
-        m[j] = v;
-    }
 }
 
 // A singleton proposes to the neighbouring aggregate of size 2..3 with the
@@ -197,17 +268,23 @@ __global__ void propose_absorption(int n, const int32_t *__restrict__ rp, const 
 }
 
 // Each target keeps its best distinct proposers, weight descending then
-// fine id ascending, up to its remaining capacity (GpuAggregation.cu:685-720).
-__global__ void accept_absorption(int coarse, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
-                                  const int32_t *__restrict__ sizes, const int32_t *__restrict__ slots,
+// fine id ascending, up to its remaining capacity (GpuAggregation.cu:685-720),
+// and takes them in: map, slots and sizes are updated in place.  A thread
+// reads only its own aggregate's size and slots (a singleton's size may turn
+// from 1 to 0 under its own thread, which has nothing to do either way), and
+// the proposals of the kernel before.
+__global__ void accept_absorption(const int32_t *count, const int32_t *__restrict__ rp,
+                                  const int32_t *__restrict__ ci, int32_t *sizes, int32_t *slots,
                                   const int32_t *__restrict__ proposal, const double *__restrict__ scores,
-                                  int32_t *__restrict__ next) {
+                                  int32_t *map) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= coarse || sizes[c] < 2 || sizes[c] >= 4) return;
+    if (c >= *count) return;
+    const int size = sizes[c];
+    if (size < 2 || size >= 4) return;
     int sel[2] = {-1, -1};
     double sw[2] = {-1, -1};
-    const int cap = 4 - sizes[c];
-    for (int k = 0; k < sizes[c]; ++k) {
+    const int cap = 4 - size;
+    for (int k = 0; k < size; ++k) {
         const int row = slots[static_cast<int64_t>(c) * 4 + k];
         for (int32_t j = rp[row]; j < rp[row + 1]; ++j) {
             const int i = ci[j];
@@ -226,24 +303,64 @@ __global__ void accept_absorption(int coarse, const int32_t *__restrict__ rp, co
             }
         }
     }
-    for (int q = 0; q < cap; ++q)
-        if (sel[q] >= 0) next[sel[q]] = c;
+    int now = size;
+    for (int q = 0; q < cap; ++q) {
+        if (sel[q] < 0) continue;
+        sizes[map[sel[q]]] = 0;
+        map[sel[q]] = c;
+        slots[static_cast<int64_t>(c) * 4 + now++] = sel[q];
+    }
+    if (now != size) sizes[c] = now;
 }
 
-__global__ void occupied(int n, const int32_t *__restrict__ sizes, int32_t *__restrict__ flags) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c <= n) flags[c] = (c < n && sizes[c] > 0) ? 1 : 0;
-}
+// Scan input: the aggregate counted under its size, 1 to 4 rows (an emptied
+// one nowhere).  The four counts give the number of aggregates and of rows
+// before one, and at the end the histogram.
+struct SizeOf {
+    const int32_t *sizes, *count;
+    __device__ Counts<4> operator()(int c) const {
+        const int s = c < *count ? sizes[c] : 0;
+        return {{s == 1, s == 2, s == 3, s == 4}};
+    }
+};
 
-// Member CSR in ascending fine order and the size histogram
-// (GpuAggregation.cu:745-757).
-__global__ void pack_members(int coarse, const int32_t *__restrict__ sizes, const int32_t *__restrict__ slots,
-                             const int32_t *__restrict__ offsets, int32_t *__restrict__ out, int32_t *histogram) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= coarse) return;
-    for (int k = 0; k < sizes[c]; ++k) out[offsets[c] + k] = slots[static_cast<int64_t>(c) * 4 + k];
-    if (sizes[c]) atomicAdd(histogram + sizes[c] - 1, 1);
-}
+// Scan output: emptied aggregates closed up (GpuAggregation.cu:745-757), the
+// members of each in ascending order and the map; position `bound` carries
+// the totals.
+struct PackAggregates {
+    int bound;
+    const int32_t *slots;
+    int32_t *off, *mem, *map, *coarse, *histogram;
+    __device__ void operator()(int c, const Counts<4> &v, const Counts<4> &before) const {
+        const auto &b = before.v;
+        const int k = b[0] + b[1] + b[2] + b[3], to = b[0] + 2 * b[1] + 3 * b[2] + 4 * b[3];
+        const int size = v.v[0] + 2 * v.v[1] + 3 * v.v[2] + 4 * v.v[3];
+        if (c == bound) {
+            *coarse = k;
+            off[k] = to;
+            for (int q = 0; q < 4; ++q) histogram[q] = b[q];
+        }
+        if (!size) return;
+        int32_t m[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            int32_t row = q < size ? slots[static_cast<int64_t>(c) * 4 + q] : INT_MAX;
+#pragma unroll
+            for (int r = 0; r <= q; ++r) {  // insertion into the sorted m[0..q)
+                const int32_t low = min(m[r], row);
+                row = max(m[r], row);
+                m[r] = low;
+            }
+        }
+        off[k] = to;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (q < size) {
+                mem[to + q] = m[q];
+                map[m[q]] = k;
+            }
+    }
+};
 
 // ---- Galerkin product by rows ----
 //
@@ -404,13 +521,27 @@ __global__ void pack_rows(int rows, const int32_t *__restrict__ base, const int3
     }
 }
 
-// sizes[coarse + 1] (zeroed sentinel) and sorted four-slot members.
-void build_members(tf_ctx *ctx, int n, int coarse, const int32_t *map, int32_t *sizes, int32_t *slots, int *overflow) {
-    memset_async(ctx, sizes, 0, (static_cast<size_t>(coarse) + 1) * sizeof(int32_t));
-    slot_members<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, map, sizes, slots, overflow);
-    launched(ctx, "slot_members");
-    sort_members<<<grid_for(coarse), kBlock, 0, ctx->stream>>>(coarse, sizes, slots);
-    launched(ctx, "sort_members");
+// Handshake rounds over vs from an empty matching; the state after them is
+// (mate, *last).
+void match_rounds(tf_ctx *ctx, const Vertices &vs, const Csr<double, int32_t> &g, int rounds, int32_t *mate,
+                  int32_t *prop0, int32_t *prop1, const int32_t **last) {
+    memset_async(ctx, mate, 0xff, static_cast<size_t>(vs.n) * sizeof(int32_t));
+    // lanes per vertex by the mean row: a lane walks 2-3 edges of a short row
+    // (4 lanes on 7-point rows read whole sectors); 32 lanes from 24 edges on
+    const int64_t mean = g.nnz / g.rows;
+    *last = nullptr;
+    for (int r = 0; r < rounds; ++r) {
+        int32_t *proposal = r & 1 ? prop1 : prop0;
+        auto go = [&](auto kernel, int lanes) {
+            kernel<<<grid_for(static_cast<int64_t>(vs.n) * lanes), kBlock, 0, ctx->stream>>>(vs, g.rp, g.ci, g.val,
+                                                                                          mate, *last, proposal);
+        };
+        if (mean < 4) go(match_round<1>, 1);
+        else if (mean < 24) go(match_round<4>, 4);
+        else go(match_round<32>, 32);
+        launched(ctx, "match_round");
+        *last = proposal;
+    }
 }
 
 }  // namespace
@@ -451,21 +582,15 @@ std::unique_ptr<tf_dcsr> strength_graph(tf_ctx *ctx, const Csr<double, int32_t> 
 int match_pairs(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, int32_t *map) {
     require(rounds >= 1 && rounds <= 8, "Invalid matching configuration");
     const int n = static_cast<int>(g.rows);
-    Temp<int32_t> mate(ctx, static_cast<size_t>(n)), proposal(ctx, static_cast<size_t>(n));
-    Temp<int32_t> flags(ctx, static_cast<size_t>(n) + 1), prefix(ctx, static_cast<size_t>(n) + 1);
-    memset_async(ctx, mate.data(), 0xff, static_cast<size_t>(n) * sizeof(int32_t));
-    for (int r = 0; r < rounds; ++r) {
-        propose<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, g.rp, g.ci, g.val, mate.data(), proposal.data());
-        launched(ctx, "propose");
-        accept<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, proposal.data(), mate.data());
-        launched(ctx, "accept");
-    }
-    roots<<<grid_for(n + 1), kBlock, 0, ctx->stream>>>(n, mate.data(), flags.data());
-    launched(ctx, "roots");
-    scan_exclusive(ctx, n + 1, flags.data(), prefix.data());
-    assign<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, mate.data(), prefix.data(), map);
-    launched(ctx, "assign");
-    return read_scalar(ctx, prefix.data() + n);
+    Temp<int32_t> mate(ctx, static_cast<size_t>(n)), prop0(ctx, static_cast<size_t>(n)),
+        prop1(ctx, static_cast<size_t>(n)), count(ctx, 1);
+    Vertices vs;
+    vs.n = n;
+    const int32_t *last = nullptr;
+    match_rounds(ctx, vs, g, rounds, mate.data(), prop0.data(), prop1.data(), &last);
+    const RootFlag root{vs, mate.data(), last};
+    scan_apply<1>(ctx, n + 1, root, AssignPairs{root, nullptr, nullptr, map, count.data()}, "assign_pairs");
+    return read_scalar(ctx, count.data());
 }
 
 std::unique_ptr<tf_dcsr> contract_graph(tf_ctx *ctx, const Csr<double, int32_t> &g, const int32_t *map, int count) {
@@ -487,64 +612,62 @@ std::unique_ptr<tf_dcsr> contract_graph(tf_ctx *ctx, const Csr<double, int32_t> 
     return compress(ctx, count, m, keys.data(), vals.data(), bits, 1);
 }
 
+// Two matchings (rows into pairs, pairs into aggregates), two absorption
+// rounds, and one compaction, in one stretch of launches: the counts stay on
+// the device until the end.
 std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, bool absorb) {
     require(rounds >= 1 && rounds <= 8 && g.rows > 0, "Invalid matching configuration");
     const int n = static_cast<int>(g.rows);
+    const size_t sn = static_cast<size_t>(n);
     auto t = std::make_unique<tf_transfer>();
     t->fine_rows = n;
-    t->map.allocate(static_cast<size_t>(n));
+    t->map.allocate(sn);
+    t->members.allocate(sn);
     int32_t *map = t->map.data();
-    const int first = match_pairs(ctx, g, rounds, map);
-    int coarse = 0;
-    {
-        auto contracted = contract_graph(ctx, g, map, first);
-        Temp<int32_t> second(ctx, static_cast<size_t>(first));
-        coarse = match_pairs(ctx, csr_of(*contracted), rounds, second.data());
-        compose<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, map, second.data());
-        launched(ctx, "compose");
-    }
-    Temp<int32_t> sizes(ctx, static_cast<size_t>(coarse) + 1), slots(ctx, static_cast<size_t>(coarse) * 4);
-    int *overflow = static_cast<int *>(ctx->arena(sizeof(int), 1));
-    memset_async(ctx, overflow, 0, sizeof(int));
-    build_members(ctx, n, coarse, map, sizes.data(), slots.data(), overflow);
+    struct Result {
+        int32_t pairs, aggregates, coarse, histogram[4];
+    };
+    Temp<Result> result(ctx, 1);
+    memset_async(ctx, result.data(), 0, sizeof(Result));
+    Result *res = result.data();
+    Temp<int32_t> mate(ctx, sn), prop0(ctx, sn), prop1(ctx, sn), lo(ctx, sn), hi(ctx, sn), sizes(ctx, sn),
+        slots(ctx, 4 * sn), off(ctx, sn + 1);
+    const int32_t *last = nullptr;
+    Vertices rows;
+    rows.n = n;
+    match_rounds(ctx, rows, g, rounds, mate.data(), prop0.data(), prop1.data(), &last);
+    const RootFlag row_root{rows, mate.data(), last};
+    scan_apply<1>(ctx, n + 1, row_root, AssignPairs{row_root, lo.data(), hi.data(), map, &res->pairs}, "assign_pairs");
+    Vertices pairs;
+    pairs.lo = lo.data();
+    pairs.hi = hi.data();
+    pairs.map = map;
+    pairs.count = &res->pairs;
+    pairs.n = n;
+    match_rounds(ctx, pairs, g, rounds, mate.data(), prop0.data(), prop1.data(), &last);
+    const RootFlag pair_root{pairs, mate.data(), last};
+    scan_apply<1>(ctx, n + 1, pair_root,
+                  AssignAggregates{pair_root, slots.data(), sizes.data(), map, &res->aggregates}, "assign_aggregates");
     if (absorb) {
-        Temp<int32_t> proposal(ctx, static_cast<size_t>(n)), next(ctx, static_cast<size_t>(n));
-        Temp<double> scores(ctx, static_cast<size_t>(n));
+        Temp<double> scores(ctx, sn);
+        int32_t *proposal = prop0.data();
         for (int round = 0; round < 2; ++round) {
             propose_absorption<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, g.rp, g.ci, g.val, map, sizes.data(),
-                                                                        proposal.data(), scores.data());
+                                                                        proposal, scores.data());
             launched(ctx, "propose_absorption");
-            copy_async(ctx, next.data(), map, static_cast<size_t>(n) * sizeof(int32_t));
-            accept_absorption<<<grid_for(coarse), kBlock, 0, ctx->stream>>>(
-                coarse, g.rp, g.ci, sizes.data(), slots.data(), proposal.data(), scores.data(), next.data());
+            accept_absorption<<<grid_for(n), kBlock, 0, ctx->stream>>>(&res->aggregates, g.rp, g.ci, sizes.data(),
+                                                                       slots.data(), proposal, scores.data(), map);
             launched(ctx, "accept_absorption");
-            copy_async(ctx, map, next.data(), static_cast<size_t>(n) * sizeof(int32_t));
-            build_members(ctx, n, coarse, map, sizes.data(), slots.data(), overflow);
         }
-        // Compact the ids of emptied aggregates.
-        Temp<int32_t> flags(ctx, static_cast<size_t>(coarse) + 1), prefix(ctx, static_cast<size_t>(coarse) + 1);
-        occupied<<<grid_for(coarse + 1), kBlock, 0, ctx->stream>>>(coarse, sizes.data(), flags.data());
-        launched(ctx, "occupied");
-        scan_exclusive(ctx, coarse + 1, flags.data(), prefix.data());
-        compose<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, map, prefix.data());
-        launched(ctx, "compose");
-        const int compacted = read_scalar(ctx, prefix.data() + coarse);
-        // The compacted table fits in the old allocation (compacted <= coarse).
-        coarse = compacted;
-        build_members(ctx, n, coarse, map, sizes.data(), slots.data(), overflow);
     }
-    if (read_scalar(ctx, overflow)) fail(TF_ERR_RUNTIME, "Aggregate capacity exceeded");
-    t->coarse_rows = coarse;
-    t->members.allocate(static_cast<size_t>(n));
-    t->offsets.allocate(static_cast<size_t>(coarse) + 1);
-    scan_exclusive(ctx, coarse + 1, sizes.data(), t->offsets.data());
-    int32_t *hist = static_cast<int32_t *>(ctx->arena(4 * sizeof(int32_t), 1));
-    memset_async(ctx, hist, 0, 4 * sizeof(int32_t));
-    pack_members<<<grid_for(coarse), kBlock, 0, ctx->stream>>>(coarse, sizes.data(), slots.data(), t->offsets.data(),
-                                                               t->members.data(), hist);
-    launched(ctx, "pack_members");
-    cuda_check(cudaMemcpyAsync(t->histogram, hist, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream),
-               "histogram readback");
+    scan_apply<4>(ctx, n + 1, SizeOf{sizes.data(), &res->aggregates},
+                  PackAggregates{n, slots.data(), off.data(), t->members.data(), map, &res->coarse, res->histogram},
+                  "pack_aggregates");
+    const Result r = read_scalar(ctx, res);
+    t->coarse_rows = r.coarse;
+    for (int k = 0; k < 4; ++k) t->histogram[k] = r.histogram[k];
+    t->offsets.allocate(static_cast<size_t>(r.coarse) + 1);
+    copy_async(ctx, t->offsets.data(), off.data(), (static_cast<size_t>(r.coarse) + 1) * sizeof(int32_t));
     cuda_check(cudaStreamSynchronize(ctx->stream), "aggregate");
     return t;
 }
