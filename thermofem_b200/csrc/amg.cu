@@ -283,13 +283,25 @@ class HierarchyImpl final : public Hierarchy {
                 break;
             }
             marks.mark(ctx, kPhStrength);
-            auto graph = strength_graph(ctx, nc, row_max.data(), o.strength_threshold);
-            if (graph->nnz == 0) {
+            TempBuffer<double> weights(ctx, static_cast<size_t>(nc.nnz));
+            TempBuffer<int> strength_flags(ctx, 1);
+            strength_weights(ctx, nc, row_max.data(), o.strength_threshold, weights.data(), strength_flags.data());
+            marks.mark(ctx, kPhAggregate);
+            auto edges = nc;
+            edges.val = weights.data();
+            int strength = 0;
+            auto t = aggregate(ctx, edges, o.matching_rounds, o.absorb_singletons != 0, strength_flags.data(),
+                               &strength);
+            if (!(strength & kStrengthSome)) {
                 stop_reason = "empty strength graph";
                 break;
             }
-            marks.mark(ctx, kPhAggregate);
-            auto t = aggregate(ctx, csr_of(*graph), o.matching_rounds, o.absorb_singletons != 0);
+            if (strength & kStrengthUnsymmetric) {
+                marks.mark(ctx, kPhStrength);
+                auto graph = strength_graph(ctx, nc, row_max.data(), o.strength_threshold);
+                marks.mark(ctx, kPhAggregate);
+                t = aggregate(ctx, csr_of(*graph), o.matching_rounds, o.absorb_singletons != 0);
+            }
             if (t->coarse_rows >= t->fine_rows) {
                 stop_reason = "no contraction";
                 break;

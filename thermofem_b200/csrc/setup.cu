@@ -11,6 +11,7 @@
 // slots are re-sorted after the atomic fill.  Sorting, reduction and scans
 // are the project's own (sort.cu).
 #include <climits>
+#include <type_traits>
 
 #include "scan.cuh"
 #include "setup.cuh"
@@ -73,6 +74,51 @@ __global__ void strength_edges(int n, const int32_t *__restrict__ rp, const int3
         }
     }
     if (!keys) count[i] = pos;
+}
+
+// Strength weights on the operator's own pattern: w[j] is the weight of edge
+// (i, c), the larger of its two directions' (GpuAggregation.cu:339-390), and
+// 0 where neither is strong and on the diagonal.  Such a graph needs no
+// sort, reduction and compaction of its own; the stages that read it skip
+// weights of 0.  flags: bit 0 some edge is strong, bit 1 a strong edge has no
+// entry for its other direction (then only the sorted graph holds it).
+// kG lanes share a row; the other direction is found by bisection in row c.
+template <int kG>
+__global__ void strength_weights_kernel(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                                        const double *__restrict__ a, const double *__restrict__ mx, double theta,
+                                        double *__restrict__ w, int *flags) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const int64_t i64 = t / kG;
+    int found = 0;
+    if (i64 < n) {
+        const int i = static_cast<int>(i64);
+        auto strong = [&](double v, double m) {
+            const double s = m > 0 ? fabs(v) / m : 0.0;
+            return m > 0 && s >= theta ? s : 0.0;
+        };
+        const double m = mx[i];
+        const int32_t end = rp[i + 1];
+        for (int32_t j = rp[i] + static_cast<int32_t>(t % kG); j < end; j += kG) {
+            const int c = ci[j];
+            double s = 0;
+            if (c != i) {
+                s = strong(a[j], m);
+                int32_t lo = rp[c], hi = rp[c + 1];
+                const int32_t last = hi;
+                while (lo < hi) {
+                    const int32_t mid = (lo + hi) >> 1;
+                    if (ci[mid] < i) lo = mid + 1;
+                    else hi = mid;
+                }
+                if (lo < last && ci[lo] == i) s = fmax(s, strong(a[lo], mx[c]));
+                else if (s > 0) found |= 2;
+                if (s > 0) found |= 1;
+            }
+            w[j] = s;
+        }
+    }
+    found = __reduce_or_sync(0xffffffffu, found);
+    if ((threadIdx.x & 31) == 0 && (found & ~*flags)) atomicOr(flags, found);
 }
 
 // The vertices of a matching: the rows themselves, or pairs of rows (lo, hi;
@@ -331,6 +377,8 @@ struct PackAggregates {
     int bound;
     const int32_t *slots;
     int32_t *off, *mem, *map, *coarse, *histogram;
+    const int *strength_flags;  // handed on to the read-back (may be null)
+    int32_t *flags;
     __device__ void operator()(int c, const Counts<4> &v, const Counts<4> &before) const {
         const auto &b = before.v;
         const int k = b[0] + b[1] + b[2] + b[3], to = b[0] + 2 * b[1] + 3 * b[2] + 4 * b[3];
@@ -339,6 +387,7 @@ struct PackAggregates {
             *coarse = k;
             off[k] = to;
             for (int q = 0; q < 4; ++q) histogram[q] = b[q];
+            *flags = strength_flags ? *strength_flags : 0;
         }
         if (!size) return;
         int32_t m[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};
@@ -521,24 +570,30 @@ __global__ void pack_rows(int rows, const int32_t *__restrict__ base, const int3
     }
 }
 
+// Calls f with the lanes that share a row, by the mean row length: a lane
+// walks two or three entries of a short row (four lanes on 7-point rows read
+// whole sectors), 32 lanes take rows of 24 entries or more.
+template <class F>
+void with_row_lanes(const Csr<double, int32_t> &a, F &&f) {
+    const int64_t mean = a.nnz / a.rows;
+    if (mean < 4) f(std::integral_constant<int, 1>{});
+    else if (mean < 24) f(std::integral_constant<int, 4>{});
+    else f(std::integral_constant<int, 32>{});
+}
+
 // Handshake rounds over vs from an empty matching; the state after them is
 // (mate, *last).
 void match_rounds(tf_ctx *ctx, const Vertices &vs, const Csr<double, int32_t> &g, int rounds, int32_t *mate,
                   int32_t *prop0, int32_t *prop1, const int32_t **last) {
     memset_async(ctx, mate, 0xff, static_cast<size_t>(vs.n) * sizeof(int32_t));
-    // lanes per vertex by the mean row: a lane walks 2-3 edges of a short row
-    // (4 lanes on 7-point rows read whole sectors); 32 lanes from 24 edges on
-    const int64_t mean = g.nnz / g.rows;
     *last = nullptr;
     for (int r = 0; r < rounds; ++r) {
         int32_t *proposal = r & 1 ? prop1 : prop0;
-        auto go = [&](auto kernel, int lanes) {
-            kernel<<<grid_for(static_cast<int64_t>(vs.n) * lanes), kBlock, 0, ctx->stream>>>(vs, g.rp, g.ci, g.val,
-                                                                                          mate, *last, proposal);
-        };
-        if (mean < 4) go(match_round<1>, 1);
-        else if (mean < 24) go(match_round<4>, 4);
-        else go(match_round<32>, 32);
+        with_row_lanes(g, [&](auto lanes) {
+            constexpr int kG = decltype(lanes)::value;
+            match_round<kG><<<grid_for(static_cast<int64_t>(vs.n) * kG), kBlock, 0, ctx->stream>>>(
+                vs, g.rp, g.ci, g.val, mate, *last, proposal);
+        });
         launched(ctx, "match_round");
         *last = proposal;
     }
@@ -579,6 +634,20 @@ std::unique_ptr<tf_dcsr> strength_graph(tf_ctx *ctx, const Csr<double, int32_t> 
     return compress(ctx, n, m, keys.data(), w.data(), bits, 1);
 }
 
+void strength_weights(tf_ctx *ctx, const Csr<double, int32_t> &a, const double *row_max, double theta, double *w,
+                      int *flags) {
+    require(std::isfinite(theta) && theta >= 0 && theta <= 1, "Invalid strength threshold");
+    require(a.nnz <= INT32_MAX / 2, "Native AMG: strength graph exceeds 32-bit capacity", TF_ERR_LENGTH);
+    const int n = static_cast<int>(a.rows);
+    memset_async(ctx, flags, 0, sizeof(int));
+    with_row_lanes(a, [&](auto lanes) {
+        constexpr int kG = decltype(lanes)::value;
+        strength_weights_kernel<kG><<<grid_for(static_cast<int64_t>(n) * kG), kBlock, 0, ctx->stream>>>(
+            n, a.rp, a.ci, a.val, row_max, theta, w, flags);
+    });
+    launched(ctx, "strength_weights");
+}
+
 int match_pairs(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, int32_t *map) {
     require(rounds >= 1 && rounds <= 8, "Invalid matching configuration");
     const int n = static_cast<int>(g.rows);
@@ -615,7 +684,8 @@ std::unique_ptr<tf_dcsr> contract_graph(tf_ctx *ctx, const Csr<double, int32_t> 
 // Two matchings (rows into pairs, pairs into aggregates), two absorption
 // rounds, and one compaction, in one stretch of launches: the counts stay on
 // the device until the end.
-std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, bool absorb) {
+std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, bool absorb,
+                                       const int *strength_flags, int *flags) {
     require(rounds >= 1 && rounds <= 8 && g.rows > 0, "Invalid matching configuration");
     const int n = static_cast<int>(g.rows);
     const size_t sn = static_cast<size_t>(n);
@@ -625,7 +695,7 @@ std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &
     t->members.allocate(sn);
     int32_t *map = t->map.data();
     struct Result {
-        int32_t pairs, aggregates, coarse, histogram[4];
+        int32_t pairs, aggregates, coarse, histogram[4], flags;
     };
     Temp<Result> result(ctx, 1);
     memset_async(ctx, result.data(), 0, sizeof(Result));
@@ -661,9 +731,11 @@ std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &
         }
     }
     scan_apply<4>(ctx, n + 1, SizeOf{sizes.data(), &res->aggregates},
-                  PackAggregates{n, slots.data(), off.data(), t->members.data(), map, &res->coarse, res->histogram},
+                  PackAggregates{n, slots.data(), off.data(), t->members.data(), map, &res->coarse, res->histogram,
+                                 strength_flags, &res->flags},
                   "pack_aggregates");
     const Result r = read_scalar(ctx, res);
+    if (flags) *flags = r.flags;
     t->coarse_rows = r.coarse;
     for (int k = 0; k < 4; ++k) t->histogram[k] = r.histogram[k];
     t->offsets.allocate(static_cast<size_t>(r.coarse) + 1);

@@ -20,7 +20,17 @@ std::unique_ptr<tf_dcsr> canonicalize(tf_ctx *ctx, const Csr<double, int32_t> &a
 std::unique_ptr<tf_dcsr> strength_graph(tf_ctx *ctx, const Csr<double, int32_t> &a, const double *row_max, double theta);
 int match_pairs(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, int32_t *map);
 std::unique_ptr<tf_dcsr> contract_graph(tf_ctx *ctx, const Csr<double, int32_t> &g, const int32_t *map, int count);
-std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, bool absorb);
+// The strength graph on a's own pattern: w[j] the weight of entry j's edge,
+// 0 where it is weak.  *flags (device): bit 0 some edge is strong; bit 1 a
+// strong edge has no entry for its other direction, and strength_graph has to
+// be taken instead.
+constexpr int kStrengthSome = 1, kStrengthUnsymmetric = 2;
+void strength_weights(tf_ctx *ctx, const Csr<double, int32_t> &a, const double *row_max, double theta, double *w,
+                      int *flags);
+// Edges of weight 0 are none.  strength_flags (device) and flags: the former's
+// value, read back with the results.
+std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, bool absorb,
+                                       const int *strength_flags = nullptr, int *flags = nullptr);
 // P^T A P for any map, by a sort over all coordinates, and for a transfer's
 // aggregates (at most four members), row by row; the same bits.
 std::unique_ptr<tf_dcsr> galerkin(tf_ctx *ctx, const Csr<double, int32_t> &a, const int32_t *map, int coarse);
