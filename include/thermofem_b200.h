@@ -328,7 +328,8 @@ int tf_amg_last_visits(const tf_amg *m, int64_t *visits, int capacity);
  * `capacity` of tf_amg_setup_phase_count() values, named by
  * tf_amg_setup_phase_name (level copies and diagonals, column and sliced
  * copies, SpMV shape tuning, strength graphs, aggregation, Galerkin
- * products, coarse LU, small-level region, layout selection). */
+ * products, coarse LU, small-level region, layout selection (always 0: no
+ * layout is timed)). */
 int tf_amg_setup_phases(const tf_amg *m, double *ms, int capacity);
 int tf_amg_setup_phase_count(void);
 const char *tf_amg_setup_phase_name(int phase);
