@@ -10,6 +10,7 @@
 // any are accepted, absorption reads the pre-round map and sizes, member
 // slots are re-sorted after the atomic fill.  Sorting, reduction and scans
 // are the project's own (sort.cu).
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 
@@ -134,17 +135,22 @@ struct Vertices {
     __device__ __forceinline__ int of(int row) const { return map ? map[row] : row; }
 };
 
-// State of a matching between rounds: mate[] (-1 unmatched) as of the
-// proposals before last, and the last round's proposals, not yet accepted:
-// a mutual pair among them is matched.  Vertex v's own thread writes that
-// into mate[v] in the next round; readers that still find -1 there come to
-// the same answer from the proposals.
-__device__ __forceinline__ int mate_of(int v, const int32_t *mate, const int32_t *last) {
-    const int m = mate[v];
-    if (m >= 0 || !last) return m;
-    const int p = last[v];
-    return p >= 0 && last[p] == v ? p : -1;
-}
+// A handshake matching in progress.  Round r works on the vertices still
+// open after round r - 1 (open[r & 1], their number in counts[r]; all of them
+// in round 0, which has no list): most vertices are matched after two rounds.
+// The order of a list is arbitrary and decides nothing.
+struct Matching {
+    Vertices vs;
+    const int32_t *rp, *ci;
+    const double *w;
+    int32_t *mate;      // -1: unmatched
+    uint8_t *taken;     // mate[v] >= 0, one byte for the proposals' gathers
+    int32_t *proposal;  // of the vertices open in the round
+    int32_t *open[2];
+    int32_t *counts;
+    __device__ __forceinline__ int size(int round) const { return round ? counts[round] : vs.size(); }
+    __device__ __forceinline__ int at(int round, int k) const { return round ? open[round & 1][k] : k; }
+};
 
 // (s, c) beats (score, best) as v's proposal (GpuAggregation.cu:402-431):
 // larger weight, then larger edge priority, then smaller vertex.
@@ -156,68 +162,92 @@ __device__ __forceinline__ bool better(int v, double s, int c, double score, int
     return a > b || (a == b && c < best);
 }
 
-// One handshake round: accepts the last round's mutual proposals
-// (GpuAggregation.cu:440-449) and writes this round's: each unmatched vertex
-// proposes its best unmatched neighbour, from one snapshot of the matching.
-// kG lanes share a vertex.
-//
-// Bound: the gathers of the neighbours' state.  Acceptance in the next
-// round's kernel halves the launches of a matching; weights are read first,
-// and only an edge that would win gathers its neighbour.
+// The proposal of open vertex v (v < 0: none), its best unmatched neighbour,
+// by kG consecutive lanes of a full warp; valid in each of them.  Weights are
+// read first: only an edge that would win gathers its neighbour.
 template <int kG>
-__global__ void match_round(Vertices vs, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
-                            const double *__restrict__ w, int32_t *mate, const int32_t *__restrict__ last,
-                            int32_t *__restrict__ proposal) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    const int lane = static_cast<int>(t % kG);
-    const int nv = vs.size();
-    if (t / kG >= nv) return;  // uniform over the vertex's lanes
-    const int v = static_cast<int>(t / kG);
-    const int mine = mate_of(v, mate, last);
-    if (mine >= 0) {
-        if (lane == 0) {
-            mate[v] = mine;
-            proposal[v] = -1;
-        }
-        return;
-    }
+__device__ __forceinline__ int propose(const Matching &m, int v, int lane) {
     int best = -1;
     double score = 0;
-    for (int k = 0; k < 2; ++k) {
-        const int row = vs.lo ? (k ? vs.hi[v] : vs.lo[v]) : (k ? -1 : v);
+    for (int part = 0; part < 2 && v >= 0; ++part) {
+        const int row = m.vs.lo ? (part ? m.vs.hi[v] : m.vs.lo[v]) : (part ? -1 : v);
         if (row < 0) break;
-        for (int32_t j = rp[row] + lane; j < rp[row + 1]; j += kG) {
-            const double s = w[j];
+        const int32_t end = m.rp[row + 1];
+        for (int32_t j = m.rp[row] + lane; j < end; j += kG) {
+            const double s = m.w[j];
             if (!(s > 0) || s < score) continue;
-            const int c = vs.of(ci[j]);
-            if (c == v || !better(v, s, c, score, best) || mate_of(c, mate, last) >= 0) continue;
+            const int c = m.vs.of(m.ci[j]);
+            if (c == v || !better(v, s, c, score, best) || m.taken[c]) continue;
             best = c;
             score = s;
         }
     }
-    if constexpr (kG > 1) {
-        const unsigned group = (kG == 32 ? 0xffffffffu : ((1u << (kG & 31)) - 1u))
-                               << ((threadIdx.x & 31) / kG * kG);
+    __syncwarp();
 #pragma unroll
-        for (int o = kG / 2; o > 0; o >>= 1) {
-            const double s = __shfl_xor_sync(group, score, o);
-            const int c = __shfl_xor_sync(group, best, o);
-            if (better(v, s, c, score, best)) {
-                best = c;
-                score = s;
+    for (int o = kG / 2; o > 0; o >>= 1) {
+        const double s = __shfl_xor_sync(0xffffffffu, score, o);
+        const int c = __shfl_xor_sync(0xffffffffu, best, o);
+        if (better(v, s, c, score, best)) {
+            best = c;
+            score = s;
+        }
+    }
+    return best;
+}
+
+// Proposals of one round, from one snapshot of the matching
+// (GpuAggregation.cu:402-431).  Bound: reading the rows of the open vertices.
+// 128^3, finest level (2.1M rows, ncu): eight rounds' proposals 277 us and
+// acceptances 137 us; visiting every vertex in every round took 980 us.
+template <int kG>
+__global__ void __launch_bounds__(kBlock) match_propose(const __grid_constant__ Matching m, int round) {
+    const int n = m.size(round), lane = threadIdx.x & 31;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * (kBlock / kG);
+    for (int64_t k0 = (blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x - lane) / kG; k0 < n; k0 += step) {
+        const int64_t k = k0 + lane / kG;
+        const int v = k < n ? m.at(round, static_cast<int>(k)) : -1;
+        const int p = propose<kG>(m, v, lane % kG);
+        if (v >= 0 && lane % kG == 0) m.proposal[v] = p;
+    }
+}
+
+// Mutual proposals become pairs (GpuAggregation.cu:440-449); the others that
+// proposed at all stay open (a vertex without a proposal never gets one).
+__device__ __forceinline__ void accept_one(const Matching &m, int round, int v) {
+    bool stays = false;
+    if (v >= 0) {
+        const int p = m.proposal[v];
+        if (p >= 0) {
+            stays = m.proposal[p] != v;
+            if (!stays) {
+                m.mate[v] = p;
+                m.taken[v] = 1;
             }
         }
     }
-    if (lane == 0) proposal[v] = best;
+    const unsigned all = __ballot_sync(0xffffffffu, stays);
+    if (!all) return;
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(m.counts + round + 1, __popc(all));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (stays) m.open[(round + 1) & 1][base + __popc(all & ((1u << lane) - 1u))] = v;
+}
+
+__global__ void __launch_bounds__(kBlock) match_accept(const __grid_constant__ Matching m, int round) {
+    const int n = m.size(round), lane = threadIdx.x & 31;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * kBlock;
+    for (int64_t k0 = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x - lane; k0 < n; k0 += step)
+        accept_one(m, round, k0 + lane < n ? m.at(round, static_cast<int>(k0) + lane) : -1);
 }
 
 // Scan input: 1 for the vertex that stands for its pair (or itself alone).
 struct RootFlag {
     Vertices vs;
-    const int32_t *mate, *last;
+    const int32_t *mate;
     __device__ Counts<1> operator()(int v) const {
         if (v >= vs.size()) return {0};
-        const int m = mate_of(v, mate, last);
+        const int m = mate[v];
         return {m < 0 || v < m ? 1 : 0};
     }
 };
@@ -231,7 +261,7 @@ struct AssignPairs {
         const int k = before.v[0];
         if (v == f.vs.n) *count = k;
         if (!flag.v[0]) return;
-        const int m = mate_of(v, f.mate, f.last);
+        const int m = f.mate[v];
         if (lo) {
             lo[k] = v;
             hi[k] = m;
@@ -256,7 +286,7 @@ struct AssignAggregates {
             slots[static_cast<int64_t>(k) * 4 + size++] = row;
             map[row] = k;
         };
-        const int m = mate_of(v, f.mate, f.last);
+        const int m = f.mate[v];
         add(f.vs.lo[v]);
         add(f.vs.hi[v]);
         if (m >= 0) {
@@ -290,12 +320,16 @@ __global__ void map_graph(int n, const int32_t *__restrict__ rp, const int32_t *
 
 // A singleton proposes to the neighbouring aggregate of size 2..3 with the
 // largest weight, ties to the smaller aggregate id (GpuAggregation.cu:646-669).
-__global__ void propose_absorption(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
-                                   const double *__restrict__ w, const int32_t *__restrict__ map,
-                                   const int32_t *__restrict__ sizes, int32_t *__restrict__ proposal,
-                                   double *__restrict__ scores) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+struct Absorption {
+    const int32_t *rp, *ci;
+    const double *w;
+    const int32_t *count;  // aggregates
+    int32_t *map, *sizes, *slots, *proposal;
+    double *scores;
+};
+
+__device__ __forceinline__ void propose_absorption(const Absorption &a, int i) {
+    const auto [rp, ci, w, count, map, sizes, slots, proposal, scores] = a;
     int best = -1;
     double score = 0;
     if (sizes[map[i]] == 1) {
@@ -319,11 +353,8 @@ __global__ void propose_absorption(int n, const int32_t *__restrict__ rp, const 
 // reads only its own aggregate's size and slots (a singleton's size may turn
 // from 1 to 0 under its own thread, which has nothing to do either way), and
 // the proposals of the kernel before.
-__global__ void accept_absorption(const int32_t *count, const int32_t *__restrict__ rp,
-                                  const int32_t *__restrict__ ci, int32_t *sizes, int32_t *slots,
-                                  const int32_t *__restrict__ proposal, const double *__restrict__ scores,
-                                  int32_t *map) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void accept_absorption(const Absorption &a, int c) {
+    const auto [rp, ci, w, count, map, sizes, slots, proposal, scores] = a;
     if (c >= *count) return;
     const int size = sizes[c];
     if (size < 2 || size >= 4) return;
@@ -357,6 +388,14 @@ __global__ void accept_absorption(const int32_t *count, const int32_t *__restric
         slots[static_cast<int64_t>(c) * 4 + now++] = sel[q];
     }
     if (now != size) sizes[c] = now;
+}
+
+__global__ void propose_absorption_kernel(int n, const __grid_constant__ Absorption a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) propose_absorption(a, i);
+}
+__global__ void accept_absorption_kernel(const __grid_constant__ Absorption a) {
+    accept_absorption(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Scan input: the aggregate counted under its size, 1 to 4 rows (an emptied
@@ -432,8 +471,8 @@ __global__ void merged_lengths(int coarse, const int32_t *__restrict__ off, cons
 }
 
 // Sorts 32 K keys held by a warp, element lane * K + r in k[r] (bitonic).
-template <int K>
-__device__ __forceinline__ void warp_sort(uint64_t (&k)[K], int lane) {
+template <int K, class Key>
+__device__ __forceinline__ void warp_sort(Key (&k)[K], int lane) {
 #pragma unroll
     for (int size = 2; size <= 32 * K; size <<= 1) {
 #pragma unroll
@@ -442,7 +481,7 @@ __device__ __forceinline__ void warp_sort(uint64_t (&k)[K], int lane) {
                 const int lx = stride / K;
 #pragma unroll
                 for (int r = 0; r < K; ++r) {
-                    const uint64_t other = __shfl_xor_sync(0xffffffffu, k[r], lx);
+                    const Key other = __shfl_xor_sync(0xffffffffu, k[r], lx);
                     const bool up = ((lane * K + r) & size) == 0, lower = (lane & lx) == 0;
                     k[r] = (up == lower) == (k[r] < other) ? k[r] : other;
                 }
@@ -451,7 +490,7 @@ __device__ __forceinline__ void warp_sort(uint64_t (&k)[K], int lane) {
                 for (int r = 0; r < K; ++r) {
                     if (r & stride) continue;
                     const bool up = ((lane * K + r) & size) == 0;
-                    const uint64_t a = k[r], b = k[r | stride];
+                    const Key a = k[r], b = k[r | stride];
                     const bool swap = up == (a > b);
                     k[r] = swap ? b : a;
                     k[r | stride] = swap ? a : b;
@@ -464,73 +503,47 @@ __device__ __forceinline__ void warp_sort(uint64_t (&k)[K], int lane) {
 // Longest merged row of merge_rows: 512 entries of 14 bytes in shared memory
 // for each of four warps.  Longer ones take the sort over all coordinates.
 constexpr int kMergeMax = 512;
+// Bits of an entry's position in a merged row of at most 32 kMax entries.
+constexpr int merge_seq_bits(int kMax) { return kMax <= 1 ? 5 : 1 + merge_seq_bits(kMax / 2); }
 
-// Row c of P^T A P (one warp): its members' entries (col = map[ci], in member
-// and entry order) sorted by (column, that order); each run of a column is
-// then added left to right, the order in which the stable sort over all
-// coordinates adds it, so the sums are the same bits.  The row goes to
-// tcol/tval from base[c], its length to count[c].
-//
-// Bound: instructions, not memory.  128^3 finest level (598k rows of 24
-// entries): 0.19 ms against 3.4 ms for map, sort, reduce and unpack.  K keys
-// per lane is the smallest power of two that holds the level's longest row.
-template <int K, int kWarps>
-__global__ void __launch_bounds__(kWarps * 32) merge_rows(int coarse, const int32_t *__restrict__ off,
-                                                          const int32_t *__restrict__ mem,
-                                                          const int32_t *__restrict__ rp,
-                                                          const int32_t *__restrict__ ci,
-                                                          const double *__restrict__ a,
-                                                          const int32_t *__restrict__ map,
-                                                          const int32_t *__restrict__ base, int32_t *__restrict__ tcol,
-                                                          double *__restrict__ tval, int32_t *__restrict__ count) {
-    constexpr int kCap = 32 * K;
-    __shared__ double s_val[kWarps][kCap];
-    __shared__ int32_t s_col[kWarps][kCap];
-    __shared__ uint16_t s_seq[kWarps][kCap];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int c = blockIdx.x * kWarps + warp;
-    if (c >= coarse) {
-        if (c == coarse && lane == 0) count[c] = 0;  // the scan's sentinel
-        return;
+// The entries of one coarse row: entry q < n is entry q + shift of A.
+struct MergeSpan {
+    int p1, p2, p3, n, s0, s1, s2, s3;
+    __device__ __forceinline__ int entry(int q) const {
+        return q + (q < p1 ? s0 : (q < p2 ? s1 : (q < p3 ? s2 : s3)));
     }
-    double *val = s_val[warp];
-    int32_t *col = s_col[warp];
-    uint16_t *seq = s_seq[warp];
-    const int o0 = off[c], members = off[c + 1] - o0;
-    int start = 0, len = 0;
-    if (lane < members) {
-        const int m = mem[o0 + lane];
-        start = rp[m];
-        len = rp[m + 1] - start;
-    }
-    const int p1 = __shfl_sync(0xffffffffu, len, 0), p2 = p1 + __shfl_sync(0xffffffffu, len, 1),
-              p3 = p2 + __shfl_sync(0xffffffffu, len, 2), n = p3 + __shfl_sync(0xffffffffu, len, 3);
-    // entry q of the merged list is entry q + shift of A within its member
-    const int s0 = __shfl_sync(0xffffffffu, start, 0), s1 = __shfl_sync(0xffffffffu, start, 1) - p1,
-              s2 = __shfl_sync(0xffffffffu, start, 2) - p2, s3 = __shfl_sync(0xffffffffu, start, 3) - p3;
-    uint64_t key[K];
+};
+
+// Merges a span of at most 32 K entries; returns the row's length (lane 31).
+template <int K, int kSeqBits, class Key>
+__device__ __forceinline__ int merge_row(const MergeSpan &m, const int32_t *__restrict__ ci,
+                                         const double *__restrict__ a, const int32_t *__restrict__ map, int lane,
+                                         double *val, int32_t *col, uint16_t *seq, int32_t *__restrict__ tcol,
+                                         double *__restrict__ tval) {
+    constexpr unsigned kSeq = (1u << kSeqBits) - 1u;
+    Key key[K];
 #pragma unroll
     for (int r = 0; r < K; ++r) {
         const int q = r * 32 + lane;
-        key[r] = ~uint64_t(0);
-        if (q < n) {
-            const int j = q + (q < p1 ? s0 : (q < p2 ? s1 : (q < p3 ? s2 : s3)));
-            key[r] = (static_cast<uint64_t>(static_cast<unsigned>(map[ci[j]])) << 16) | static_cast<unsigned>(q);
+        key[r] = static_cast<Key>(~Key(0));
+        if (q < m.n) {
+            const int j = m.entry(q);
+            key[r] = (static_cast<Key>(static_cast<unsigned>(map[ci[j]])) << kSeqBits) | static_cast<unsigned>(q);
             val[q] = a[j];
         }
     }
     warp_sort<K>(key, lane);
-    const uint64_t before = __shfl_up_sync(0xffffffffu, key[K - 1], 1);
+    const Key before = __shfl_up_sync(0xffffffffu, key[K - 1], 1);
     unsigned heads = 0;
 #pragma unroll
     for (int r = 0; r < K; ++r) {
         const int e = lane * K + r;
-        if (e < n) {
-            const int32_t mine = static_cast<int32_t>(key[r] >> 16);
+        if (e < m.n) {
+            const int32_t mine = static_cast<int32_t>(key[r] >> kSeqBits);
             col[e] = mine;
-            seq[e] = static_cast<uint16_t>(key[r] & 0xffffu);
-            const uint64_t left = r > 0 ? key[r > 0 ? r - 1 : 0] : before;
-            if (e == 0 || static_cast<int32_t>(left >> 16) != mine) heads |= 1u << r;
+            seq[e] = static_cast<uint16_t>(key[r] & kSeq);
+            const Key left = r > 0 ? key[r > 0 ? r - 1 : 0] : before;
+            if (e == 0 || static_cast<int32_t>(left >> kSeqBits) != mine) heads |= 1u << r;
         }
     }
     __syncwarp();
@@ -540,19 +553,83 @@ __global__ void __launch_bounds__(kWarps * 32) merge_rows(int coarse, const int3
         const int y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += y;
     }
-    if (lane == 31) count[c] = inc;
-    int out = base[c] + inc - own;
+    int out = inc - own;
 #pragma unroll
     for (int r = 0; r < K; ++r) {
         if (!(heads >> r & 1u)) continue;
         const int e = lane * K + r;
         const int32_t mine = col[e];
         double sum = val[seq[e]];
-        for (int q = e + 1; q < n && col[q] == mine; ++q) sum += val[seq[q]];
+        for (int q = e + 1; q < m.n && col[q] == mine; ++q) sum += val[seq[q]];
         tcol[out] = mine;
         tval[out] = sum;
         ++out;
     }
+    return inc;
+}
+
+// Row c of P^T A P (one warp): its members' entries (col = map[ci], in member
+// and entry order) sorted by (column, that order); each run of a column is
+// then added left to right, the order in which the stable sort over all
+// coordinates adds it, so the sums are the same bits.  The row goes to
+// tcol/tval from base[c], its length to count[c].
+//
+// Bound: the sort's instructions, not memory.  Each row is sorted in the
+// smallest power of two that holds it (kMax: the level's longest row), with
+// 32-bit keys where the coarse column and the position fit one.  128^3 (ncu):
+// finest level, 598k rows of 24 entries, 0.28 ms; the other eight levels
+// together 0.22 ms, 0.39 ms with every row sorted as the longest.  Map, sort,
+// reduce and unpack took 3.4 ms on the finest level.
+template <int kMax, int kWarps, class Key>
+__global__ void __launch_bounds__(kWarps * 32) merge_rows(int coarse, const int32_t *__restrict__ off,
+                                                          const int32_t *__restrict__ mem,
+                                                          const int32_t *__restrict__ rp,
+                                                          const int32_t *__restrict__ ci,
+                                                          const double *__restrict__ a,
+                                                          const int32_t *__restrict__ map,
+                                                          const int32_t *__restrict__ base, int32_t *__restrict__ tcol,
+                                                          double *__restrict__ tval, int32_t *__restrict__ count) {
+    constexpr int kCap = 32 * kMax;
+    __shared__ double s_val[kWarps][kCap];
+    __shared__ int32_t s_col[kWarps][kCap];
+    __shared__ uint16_t s_seq[kWarps][kCap];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x * kWarps + warp;
+    if (c >= coarse) {
+        if (c == coarse && lane == 0) count[c] = 0;  // the scan's sentinel
+        return;
+    }
+    const int o0 = off[c], members = off[c + 1] - o0;
+    int start = 0, len = 0;
+    if (lane < members) {
+        const int row = mem[o0 + lane];
+        start = rp[row];
+        len = rp[row + 1] - start;
+    }
+    MergeSpan m;
+    m.p1 = __shfl_sync(0xffffffffu, len, 0);
+    m.p2 = m.p1 + __shfl_sync(0xffffffffu, len, 1);
+    m.p3 = m.p2 + __shfl_sync(0xffffffffu, len, 2);
+    m.n = m.p3 + __shfl_sync(0xffffffffu, len, 3);
+    m.s0 = __shfl_sync(0xffffffffu, start, 0);
+    m.s1 = __shfl_sync(0xffffffffu, start, 1) - m.p1;
+    m.s2 = __shfl_sync(0xffffffffu, start, 2) - m.p2;
+    m.s3 = __shfl_sync(0xffffffffu, start, 3) - m.p3;
+    auto merge = [&](auto k) {
+        constexpr int K = decltype(k)::value;
+        const int32_t to = base[c];
+        const int n = merge_row<K, merge_seq_bits(kMax), Key>(m, ci, a, map, lane, s_val[warp], s_col[warp], s_seq[warp], tcol + to,
+                                        tval + to);
+        if (lane == 31) count[c] = n;
+    };
+    if (m.n <= 32) return merge(std::integral_constant<int, 1>{});
+    if constexpr (kMax >= 2)
+        if (m.n <= 64) return merge(std::integral_constant<int, 2>{});
+    if constexpr (kMax >= 4)
+        if (m.n <= 128) return merge(std::integral_constant<int, 4>{});
+    if constexpr (kMax >= 8)
+        if (m.n <= 256) return merge(std::integral_constant<int, 8>{});
+    if constexpr (kMax >= 16) merge(std::integral_constant<int, 16>{});
 }
 
 // The merged rows moved together: row c's entries from base[c] to rp[c]
@@ -581,21 +658,106 @@ void with_row_lanes(const Csr<double, int32_t> &a, F &&f) {
     else f(std::integral_constant<int, 32>{});
 }
 
-// Handshake rounds over vs from an empty matching; the state after them is
-// (mate, *last).
-void match_rounds(tf_ctx *ctx, const Vertices &vs, const Csr<double, int32_t> &g, int rounds, int32_t *mate,
-                  int32_t *prop0, int32_t *prop1, const int32_t **last) {
-    memset_async(ctx, mate, 0xff, static_cast<size_t>(vs.n) * sizeof(int32_t));
-    *last = nullptr;
+// Every stage of an aggregation, for the launches below and the one-CTA
+// kernel.
+struct AggregateState {
+    int n, rounds;
+    bool absorb;
+    Matching rows, pairs;
+    AssignPairs to_pairs;
+    AssignAggregates to_aggregates;
+    Absorption absorption;
+    SizeOf size_of;
+    PackAggregates pack;
+};
+
+// One CTA runs the whole aggregation of a small level: at 2 us and more per
+// dependent launch, 45 launches cost more than one SM's work on a few
+// thousand rows.  Its stages are separated by __syncthreads (global memory
+// written by the CTA is visible to it after one).
+constexpr int kAggregateOneCta = 4096, kAggregateOneCtaEntries = 65536;  // rows, entries
+
+template <int kG>
+__device__ void match_in_block(const Matching &m, int rounds) {
+    const int lane = threadIdx.x & 31, nt = blockDim.x;
+    const int nv = m.vs.size();
+    for (int v = threadIdx.x; v < nv; v += nt) {
+        m.mate[v] = -1;
+        m.taken[v] = 0;
+    }
+    for (int r = threadIdx.x; r <= rounds; r += nt) m.counts[r] = 0;
+    __syncthreads();
+    for (int round = 0; round < rounds; ++round) {
+        const int n = round ? *const_cast<volatile int32_t *>(m.counts + round) : nv;
+        if (n == 0) break;
+        for (int k0 = (threadIdx.x - lane) / kG; k0 < n; k0 += nt / kG) {
+            const int k = k0 + lane / kG;
+            const int v = k < n ? m.at(round, k) : -1;
+            const int p = propose<kG>(m, v, lane % kG);
+            if (v >= 0 && lane % kG == 0) m.proposal[v] = p;
+        }
+        __syncthreads();
+        for (int k0 = threadIdx.x - lane; k0 < n; k0 += nt)
+            accept_one(m, round, k0 + lane < n ? m.at(round, k0 + lane) : -1);
+        __syncthreads();
+    }
+}
+
+template <int N, class In, class Out>
+__device__ void scan_in_block(int n, const In &in, const Out &out) {
+    using namespace scan_detail;
+    Counts<N> carry{};
+    for (int first = 0; first < n; first += kMidThreads * kItems)
+        scan_tile<N, kMidThreads>(first, n, in, out, carry);
+    __syncthreads();
+}
+
+template <int kG>
+__global__ void __launch_bounds__(scan_detail::kMidThreads) aggregate_one_cta(const __grid_constant__ AggregateState s) {
+    match_in_block<kG>(s.rows, s.rounds);
+    scan_in_block<1>(s.n + 1, s.to_pairs.f, s.to_pairs);
+    match_in_block<kG>(s.pairs, s.rounds);
+    scan_in_block<1>(s.n + 1, s.to_aggregates.f, s.to_aggregates);
+    for (int round = 0; s.absorb && round < 2; ++round) {
+        for (int i = threadIdx.x; i < s.n; i += blockDim.x) propose_absorption(s.absorption, i);
+        __syncthreads();
+        for (int c = threadIdx.x; c < s.n; c += blockDim.x) accept_absorption(s.absorption, c);
+        __syncthreads();
+    }
+    scan_in_block<4>(s.n + 1, s.size_of, s.pack);
+}
+
+// Temporary arrays of a matching over at most n vertices.
+struct MatchBuffers {
+    Temp<int32_t> mate, proposal, open0, open1, counts;
+    Temp<uint8_t> taken;
+    MatchBuffers(tf_ctx *ctx, int n, int rounds)
+        : mate(ctx, static_cast<size_t>(n)), proposal(ctx, static_cast<size_t>(n)),
+          open0(ctx, static_cast<size_t>(n)), open1(ctx, static_cast<size_t>(n)),
+          counts(ctx, static_cast<size_t>(rounds) + 1), taken(ctx, static_cast<size_t>(n)) {}
+    Matching matching(const Vertices &vs, const Csr<double, int32_t> &g) const {
+        return {vs, g.rp, g.ci, g.val, mate.data(), taken.data(), proposal.data(), {open0.data(), open1.data()},
+                counts.data()};
+    }
+};
+
+// Handshake rounds from an empty matching, two launches each.
+void match_rounds(tf_ctx *ctx, const Matching &m, const Csr<double, int32_t> &g, int rounds) {
+    memset_async(ctx, m.mate, 0xff, static_cast<size_t>(m.vs.n) * sizeof(int32_t));
+    memset_async(ctx, m.taken, 0, static_cast<size_t>(m.vs.n));
+    memset_async(ctx, m.counts, 0, (static_cast<size_t>(rounds) + 1) * sizeof(int32_t));
+    // later rounds: an unknown, smaller number of vertices, in a grid stride
+    const unsigned most = static_cast<unsigned>(ctx->sm_count) * 8;
     for (int r = 0; r < rounds; ++r) {
-        int32_t *proposal = r & 1 ? prop1 : prop0;
         with_row_lanes(g, [&](auto lanes) {
             constexpr int kG = decltype(lanes)::value;
-            match_round<kG><<<grid_for(static_cast<int64_t>(vs.n) * kG), kBlock, 0, ctx->stream>>>(
-                vs, g.rp, g.ci, g.val, mate, *last, proposal);
+            const unsigned grid = grid_for(static_cast<int64_t>(m.vs.n) * kG);
+            match_propose<kG><<<r ? std::min(grid, most) : grid, kBlock, 0, ctx->stream>>>(m, r);
         });
-        launched(ctx, "match_round");
-        *last = proposal;
+        launched(ctx, "match_propose");
+        const unsigned grid = grid_for(m.vs.n);
+        match_accept<<<r ? std::min(grid, most) : grid, kBlock, 0, ctx->stream>>>(m, r);
+        launched(ctx, "match_accept");
     }
 }
 
@@ -651,13 +813,13 @@ void strength_weights(tf_ctx *ctx, const Csr<double, int32_t> &a, const double *
 int match_pairs(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, int32_t *map) {
     require(rounds >= 1 && rounds <= 8, "Invalid matching configuration");
     const int n = static_cast<int>(g.rows);
-    Temp<int32_t> mate(ctx, static_cast<size_t>(n)), prop0(ctx, static_cast<size_t>(n)),
-        prop1(ctx, static_cast<size_t>(n)), count(ctx, 1);
+    MatchBuffers buffers(ctx, n, rounds);
+    Temp<int32_t> count(ctx, 1);
     Vertices vs;
     vs.n = n;
-    const int32_t *last = nullptr;
-    match_rounds(ctx, vs, g, rounds, mate.data(), prop0.data(), prop1.data(), &last);
-    const RootFlag root{vs, mate.data(), last};
+    const Matching m = buffers.matching(vs, g);
+    match_rounds(ctx, m, g, rounds);
+    const RootFlag root{vs, m.mate};
     scan_apply<1>(ctx, n + 1, root, AssignPairs{root, nullptr, nullptr, map, count.data()}, "assign_pairs");
     return read_scalar(ctx, count.data());
 }
@@ -682,8 +844,7 @@ std::unique_ptr<tf_dcsr> contract_graph(tf_ctx *ctx, const Csr<double, int32_t> 
 }
 
 // Two matchings (rows into pairs, pairs into aggregates), two absorption
-// rounds, and one compaction, in one stretch of launches: the counts stay on
-// the device until the end.
+// rounds and one compaction: the counts stay on the device until the end.
 std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, bool absorb,
                                        const int *strength_flags, int *flags) {
     require(rounds >= 1 && rounds <= 8 && g.rows > 0, "Invalid matching configuration");
@@ -700,40 +861,47 @@ std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &
     Temp<Result> result(ctx, 1);
     memset_async(ctx, result.data(), 0, sizeof(Result));
     Result *res = result.data();
-    Temp<int32_t> mate(ctx, sn), prop0(ctx, sn), prop1(ctx, sn), lo(ctx, sn), hi(ctx, sn), sizes(ctx, sn),
-        slots(ctx, 4 * sn), off(ctx, sn + 1);
-    const int32_t *last = nullptr;
-    Vertices rows;
+    MatchBuffers buffers(ctx, n, rounds);
+    Temp<int32_t> lo(ctx, sn), hi(ctx, sn), sizes(ctx, sn), slots(ctx, 4 * sn), off(ctx, sn + 1);
+    Temp<double> scores(ctx, absorb ? sn : 0);
+    Vertices rows, pairs;
     rows.n = n;
-    match_rounds(ctx, rows, g, rounds, mate.data(), prop0.data(), prop1.data(), &last);
-    const RootFlag row_root{rows, mate.data(), last};
-    scan_apply<1>(ctx, n + 1, row_root, AssignPairs{row_root, lo.data(), hi.data(), map, &res->pairs}, "assign_pairs");
-    Vertices pairs;
     pairs.lo = lo.data();
     pairs.hi = hi.data();
     pairs.map = map;
     pairs.count = &res->pairs;
     pairs.n = n;
-    match_rounds(ctx, pairs, g, rounds, mate.data(), prop0.data(), prop1.data(), &last);
-    const RootFlag pair_root{pairs, mate.data(), last};
-    scan_apply<1>(ctx, n + 1, pair_root,
-                  AssignAggregates{pair_root, slots.data(), sizes.data(), map, &res->aggregates}, "assign_aggregates");
-    if (absorb) {
-        Temp<double> scores(ctx, sn);
-        int32_t *proposal = prop0.data();
-        for (int round = 0; round < 2; ++round) {
-            propose_absorption<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, g.rp, g.ci, g.val, map, sizes.data(),
-                                                                        proposal, scores.data());
+    AggregateState s;
+    s.n = n;
+    s.rounds = rounds;
+    s.absorb = absorb;
+    s.rows = buffers.matching(rows, g);
+    s.pairs = buffers.matching(pairs, g);
+    s.to_pairs = {{rows, s.rows.mate}, lo.data(), hi.data(), map, &res->pairs};
+    s.to_aggregates = {{pairs, s.pairs.mate}, slots.data(), sizes.data(), map, &res->aggregates};
+    s.absorption = {g.rp, g.ci, g.val, &res->aggregates, map, sizes.data(), slots.data(), s.rows.proposal,
+                    scores.data()};
+    s.size_of = {sizes.data(), &res->aggregates};
+    s.pack = {n, slots.data(), off.data(), t->members.data(), map, &res->coarse, res->histogram, strength_flags,
+              &res->flags};
+    if (n <= kAggregateOneCta && g.nnz <= kAggregateOneCtaEntries) {
+        with_row_lanes(g, [&](auto lanes) {
+            aggregate_one_cta<decltype(lanes)::value><<<1, scan_detail::kMidThreads, 0, ctx->stream>>>(s);
+        });
+        launched(ctx, "aggregate_one_cta");
+    } else {
+        match_rounds(ctx, s.rows, g, rounds);
+        scan_apply<1>(ctx, n + 1, s.to_pairs.f, s.to_pairs, "assign_pairs");
+        match_rounds(ctx, s.pairs, g, rounds);
+        scan_apply<1>(ctx, n + 1, s.to_aggregates.f, s.to_aggregates, "assign_aggregates");
+        for (int round = 0; absorb && round < 2; ++round) {
+            propose_absorption_kernel<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, s.absorption);
             launched(ctx, "propose_absorption");
-            accept_absorption<<<grid_for(n), kBlock, 0, ctx->stream>>>(&res->aggregates, g.rp, g.ci, sizes.data(),
-                                                                       slots.data(), proposal, scores.data(), map);
+            accept_absorption_kernel<<<grid_for(n), kBlock, 0, ctx->stream>>>(s.absorption);
             launched(ctx, "accept_absorption");
         }
+        scan_apply<4>(ctx, n + 1, s.size_of, s.pack, "pack_aggregates");
     }
-    scan_apply<4>(ctx, n + 1, SizeOf{sizes.data(), &res->aggregates},
-                  PackAggregates{n, slots.data(), off.data(), t->members.data(), map, &res->coarse, res->histogram,
-                                 strength_flags, &res->flags},
-                  "pack_aggregates");
     const Result r = read_scalar(ctx, res);
     if (flags) *flags = r.flags;
     t->coarse_rows = r.coarse;
@@ -769,17 +937,24 @@ std::unique_ptr<tf_dcsr> galerkin(tf_ctx *ctx, const Csr<double, int32_t> &a, co
     if (most > kMergeMax) return galerkin(ctx, a, map, coarse);
     Temp<int32_t> tcol(ctx, static_cast<size_t>(a.nnz));
     Temp<double> tval(ctx, static_cast<size_t>(a.nnz));
-    auto merge = [&](auto kernel, int warps) {
-        kernel<<<grid_for(coarse + 1, warps), warps * 32, 0, ctx->stream>>>(coarse, off, mem, a.rp, a.ci, a.val, map,
-                                                                            base.data(), tcol.data(), tval.data(),
-                                                                            count.data());
+    auto merge = [&](auto kmax, auto warps) {
+        constexpr int kMax = decltype(kmax)::value, kWarps = decltype(warps)::value;
+        auto go = [&](auto kernel) {
+            kernel<<<grid_for(coarse + 1, kWarps), kWarps * 32, 0, ctx->stream>>>(coarse, off, mem, a.rp, a.ci, a.val,
+                                                                                  map, base.data(), tcol.data(),
+                                                                                  tval.data(), count.data());
+        };
+        // (31 bits: no key equals the padding key)
+        if (column_bits(coarse) + merge_seq_bits(kMax) <= 31) go(merge_rows<kMax, kWarps, uint32_t>);
+        else go(merge_rows<kMax, kWarps, uint64_t>);
         launched(ctx, "merge_rows");
     };
-    if (most <= 32) merge(merge_rows<1, 8>, 8);
-    else if (most <= 64) merge(merge_rows<2, 8>, 8);
-    else if (most <= 128) merge(merge_rows<4, 8>, 8);
-    else if (most <= 256) merge(merge_rows<8, 8>, 8);
-    else merge(merge_rows<16, 4>, 4);
+    using std::integral_constant;
+    if (most <= 32) merge(integral_constant<int, 1>{}, integral_constant<int, 8>{});
+    else if (most <= 64) merge(integral_constant<int, 2>{}, integral_constant<int, 8>{});
+    else if (most <= 128) merge(integral_constant<int, 4>{}, integral_constant<int, 8>{});
+    else if (most <= 256) merge(integral_constant<int, 8>{}, integral_constant<int, 8>{});
+    else merge(integral_constant<int, 16>{}, integral_constant<int, 4>{});
     auto out = std::make_unique<tf_dcsr>();
     out->rows = out->cols = coarse;
     out->offsets.allocate(static_cast<size_t>(coarse + 1) * sizeof(int32_t));
