@@ -112,6 +112,9 @@ class TailRegion {
     size_t shared_bytes() const { return smem_; }
 
   private:
+    bool plan_one_cta(tf_ctx *ctx, const std::vector<TailLevel<S>> &levels, const TailParent &parent,
+                      const std::vector<std::vector<int32_t>> &rps, const std::vector<std::vector<int32_t>> &offs,
+                      const double *inv, int dense_n, S w, int max_steps, size_t limit);
     struct Step {
         int op, level, a, b, c;
     };
