@@ -106,9 +106,28 @@ __global__ void forward_kernel(int64_t n, const float *__restrict__ x, const uin
     }
 }
 
+// Sums of 32 values over the 32 lanes at once: lane l returns the sum of
+// g[l].  Each exchange halves the values a lane still carries (31 shuffles
+// instead of five per value); the pairs added are those of a shuffle-down
+// tree, whose lane 0 has the same bits.
+__device__ __forceinline__ float sum_each(float (&g)[32], int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float keep = upper ? g[i + o] : g[i], send = upper ? g[i] : g[i + o];
+            g[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return g[0];
+}
+
 // Per-CTA sums of the gradient of sum_i (omega_i - t_i)^2 and of the loss:
-// each warp reduces its 32 rows per parameter with shuffles, lane 0 adds the
-// warp sum to its slot, and the slots are added in warp order.
+// each warp reduces its 32 rows per parameter with shuffles and adds the
+// warp sum to its slot; the slots are added in warp order.  Bound: the
+// shuffles of the 194 sums, which sum_each cut from 970 to 196 per 32 rows
+// (32,768 rows: 11.7 -> 6.8 us, ncu).
 __global__ void __launch_bounds__(kMlpBlock) backward_kernel(int64_t n, const float *__restrict__ x,
                                                              const float *__restrict__ target,
                                                              const uint16_t *__restrict__ bf, float lo, float hi,
@@ -148,15 +167,21 @@ __global__ void __launch_bounds__(kMlpBlock) backward_kernel(int64_t n, const fl
         };
         add(kP, e * e);
         add(kB2, dz);
+        static_assert(kH == 32 && kF == 4, "32 sums at a time");
+        float g[32], dh[kH];
 #pragma unroll
         for (int j = 0; j < kH; ++j) {
-            const float h = fmaxf(a[j], 0.0f);
-            add(kW2 + j, dz * h);
-            const float dh = a[j] > 0.0f ? dz * sp[kW2 + j] : 0.0f;
-            add(kB1 + j, dh);
-#pragma unroll
-            for (int k = 0; k < kF; ++k) add(kW1 + j * kF + k, dh * xv[k]);
+            g[j] = dz * fmaxf(a[j], 0.0f);
+            dh[j] = a[j] > 0.0f ? dz * sp[kW2 + j] : 0.0f;
         }
+        slot[warp][kW2 + lane] += static_cast<double>(sum_each(g, lane));
+#pragma unroll
+        for (int j0 = 0; j0 < kH; j0 += 8) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) g[k] = dh[j0 + k / kF] * xv[k % kF];
+            slot[warp][kW1 + j0 * kF + lane] += static_cast<double>(sum_each(g, lane));
+        }
+        slot[warp][kB1 + lane] += static_cast<double>(sum_each(dh, lane));
     }
     __syncthreads();
     for (int k = threadIdx.x; k < kGradSlots; k += blockDim.x) {
@@ -166,14 +191,26 @@ __global__ void __launch_bounds__(kMlpBlock) backward_kernel(int64_t n, const fl
     }
 }
 
-// grad[k] += sum over CTAs of partial[cta][k], in CTA order.
+// grad[k] += sum over CTAs of partial[cta][k], in CTA order, 64 loads in
+// flight, a warp per 32 sums; grad[kP + 1] = what this added to the loss sum.
 __global__ void gradient_sum_kernel(int parts, const double *__restrict__ partial, double *__restrict__ grad) {
     pdl_enter();
-    for (int k = threadIdx.x; k < kGradSlots; k += blockDim.x) {
-        double v = 0.0;
-        for (int c = 0; c < parts; ++c) v += partial[static_cast<int64_t>(c) * kGradSlots + k];
-        grad[k] += v;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= kGradSlots) return;
+    constexpr int kAhead = 64;
+    double v = 0.0;
+    for (int c0 = 0; c0 < parts; c0 += kAhead) {
+        double t[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            t[u] = c0 + u < parts ? partial[static_cast<int64_t>(c0 + u) * kGradSlots + k] : 0.0;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (c0 + u < parts) v += t[u];
     }
+    const double before = grad[k], after = before + v;
+    grad[k] = after;
+    if (k == kP) grad[kP + 1] = after - before;
 }
 
 // Momentum SGD on the FP32 master weights with the mean gradient of the
@@ -334,7 +371,7 @@ int tf_mlp_create(tf_ctx *ctx, uint64_t seed, double omega_min, double omega_max
         m->params.allocate(kP);
         m->velocity.allocate(kP);
         m->bf16.allocate(kP);
-        m->grad.allocate(kGradSlots);
+        m->grad.allocate(kGradSlots + 1);
         m->partial.allocate(static_cast<size_t>(kMaxGrid) * kGradSlots);
         memset_async(ctx, m->velocity.data(), 0, kP * sizeof(float));
         memset_async(ctx, m->grad.data(), 0, kGradSlots * sizeof(double));
@@ -416,13 +453,12 @@ int tf_mlp_backward(tf_mlp *m, int64_t n, const float *features, const float *ta
         DeviceScope scope(m->ctx->device);
         tf_ctx *ctx = m->ctx;
         const unsigned g = grid_rows(n);
-        const double before = loss ? read_scalar(ctx, m->grad.data() + kP) : 0.0;
         launch_kernel(ctx, "mlp_backward", backward_kernel, g, kMlpBlock, 0, n, features, target,
                       static_cast<const uint16_t *>(m->bf16.data()), m->omega_min, m->omega_max, m->partial.data());
-        launch_kernel(ctx, "mlp_gradient_sum", gradient_sum_kernel, 1, kMlpBlock, 0, static_cast<int>(g),
+        launch_kernel(ctx, "mlp_gradient_sum", gradient_sum_kernel, grid_for(kGradSlots, 32), 32, 0, static_cast<int>(g),
                       static_cast<const double *>(m->partial.data()), m->grad.data());
         m->rows += static_cast<double>(n);
-        if (loss) *loss = (read_scalar(ctx, m->grad.data() + kP) - before) / static_cast<double>(n);
+        if (loss) *loss = read_scalar(ctx, m->grad.data() + kP + 1) / static_cast<double>(n);
     });
 }
 
@@ -446,7 +482,6 @@ int tf_mlp_sgd(tf_mlp *m, double lr, double momentum) {
         launch_kernel(m->ctx, "mlp_sgd", sgd_kernel, 1, kMlpBlock, 0, m->params.data(), m->velocity.data(),
                       m->grad.data(), m->rows, static_cast<float>(lr), static_cast<float>(momentum), m->bf16.data());
         m->rows = 0;
-        cuda_check(cudaStreamSynchronize(m->ctx->stream), "sgd");
     });
 }
 
