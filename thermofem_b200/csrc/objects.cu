@@ -28,6 +28,8 @@ struct tf_jacobi {
     int64_t n{0}, nnz{0};
     DeviceBuffer<int32_t> rp, ci;
     DeviceBuffer<unsigned char> val, dinv, rhs, x0, x1;
+    SlicedCopy<float> banded32;  // stencil operators: the copy the sweeps stream instead of rp, ci, val
+    SlicedCopy<double> banded64;
 };
 
 struct tf_solver {
@@ -56,6 +58,22 @@ namespace {
 void check_types(int value_type, int index_type) {
     require(value_type == TF_F32 || value_type == TF_F64, "value type must be TF_F32 or TF_F64");
     require(index_type == TF_I32 || index_type == TF_I64, "index type must be TF_I32 or TF_I64");
+}
+
+// Memory that kernels on this device may read and write.
+bool on_device(const void *p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    int device = 0;
+    return a.type == cudaMemoryTypeDevice && cudaGetDevice(&device) == cudaSuccess && a.device == device;
+}
+
+bool disjoint(const void *a, const void *b, size_t bytes) {
+    const auto pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);
+    return pa + bytes <= pb || pb + bytes <= pa;
 }
 
 // After a component's buffers were freed (in the order of the context's
@@ -146,8 +164,7 @@ int tf_amg_apply(tf_amg *m, const void *rhs, void *x) {
             m->h->apply(m->ctx, static_cast<const double *>(rhs), static_cast<double *>(x));
         else
             m->h->apply(m->ctx, static_cast<const float *>(rhs), static_cast<float *>(x));
-        cuda_check(cudaStreamSynchronize(m->ctx->stream), "AMG apply");
-        check_faults(m->ctx);
+        check_faults(m->ctx);  // (synchronises the stream)
     });
 }
 
@@ -316,17 +333,24 @@ int tf_jacobi_setup(tf_jacobi *j, const tf_csr *a) {
         const auto nc = csr_of(*native);
         copy_async(ctx, rp.data(), nc.rp, (n + 1) * 4);
         copy_async(ctx, ci.data(), nc.ci, nnz * 4);
-        if (j->value_type == TF_F64) {
-            convert(ctx, nnz, nc.val, reinterpret_cast<double *>(val.data()));
-            Csr<double, int32_t> c{n, n, nnz, rp.data(), ci.data(), reinterpret_cast<const double *>(val.data())};
-            inverse_diagonal(ctx, c, reinterpret_cast<double *>(dinv.data()));
-        } else {
-            convert(ctx, nnz, nc.val, reinterpret_cast<float *>(val.data()));
-            Csr<float, int32_t> c{n, n, nnz, rp.data(), ci.data(), reinterpret_cast<const float *>(val.data())};
-            inverse_diagonal(ctx, c, reinterpret_cast<float *>(dinv.data()));
-        }
+        SlicedCopy<float> banded32;
+        SlicedCopy<double> banded64;
         DeviceBuffer<unsigned char> rhs(static_cast<size_t>(n) * vs), x0(static_cast<size_t>(n) * vs),
             x1(static_cast<size_t>(n) * vs);
+        auto prepare = [&](auto t, auto &banded) {
+            using T = decltype(t);
+            convert(ctx, nnz, nc.val, reinterpret_cast<T *>(val.data()));
+            Csr<T, int32_t> c{n, n, nnz, rp.data(), ci.data(), reinterpret_cast<const T *>(val.data())};
+            inverse_diagonal(ctx, c, reinterpret_cast<T *>(dinv.data()));
+            // 8.25 instead of 12 bytes an entry (FP64), the same bits
+            if (sliced_enabled() && banded_enabled() && build_banded(ctx, c, banded)) {
+                banded.attach(c);
+                fill_zero(ctx, n, reinterpret_cast<T *>(x0.data()));
+                tune_spmv(ctx, c, reinterpret_cast<const T *>(x0.data()), reinterpret_cast<T *>(x1.data()));
+            }
+        };
+        if (j->value_type == TF_F64) prepare(double{}, banded64);
+        else prepare(float{}, banded32);
         cuda_check(cudaStreamSynchronize(ctx->stream), "Jacobi setup");
         j->n = n;
         j->nnz = nnz;
@@ -337,6 +361,8 @@ int tf_jacobi_setup(tf_jacobi *j, const tf_csr *a) {
         j->rhs = std::move(rhs);
         j->x0 = std::move(x0);
         j->x1 = std::move(x1);
+        j->banded32 = std::move(banded32);
+        j->banded64 = std::move(banded64);
         j->ready = true;
     });
 }
@@ -349,23 +375,36 @@ int tf_jacobi_apply(tf_jacobi *j, const void *rhs, void *x) {
         DeviceScope scope(j->ctx->device);
         tf_ctx *ctx = j->ctx;
         const size_t bytes = static_cast<size_t>(j->n) * type_size(j->value_type);
-        copy_async(ctx, j->rhs.data(), rhs, bytes);
-        copy_async(ctx, j->x0.data(), x, bytes);
-        auto run = [&](auto t) {
+        // Device vectors that do not overlap are read and written where they
+        // are; others (host memory, rhs aliasing x) go through the component's
+        // own: three copies of the vectors, 15 us at 885k rows in FP64.
+        const bool direct = on_device(rhs) && on_device(x) && disjoint(rhs, x, bytes);
+        auto run = [&](auto t, const auto &banded) {
             using T = decltype(t);
             Csr<T, int32_t> c{j->n, j->n, j->nnz, j->rp.data(), j->ci.data(), reinterpret_cast<const T *>(j->val.data())};
-            T *xa = reinterpret_cast<T *>(j->x0.data()), *xb = reinterpret_cast<T *>(j->x1.data());
-            for (int s = 0; s < j->sweeps; ++s) {
-                jacobi_sweep(ctx, c, reinterpret_cast<const T *>(j->dinv.data()), reinterpret_cast<const T *>(j->rhs.data()),
-                             xa, xb, static_cast<T>(j->weight), nullptr, nullptr, static_cast<const T *>(nullptr));
-                std::swap(xa, xb);
+            banded.attach(c);
+            T *own[2] = {reinterpret_cast<T *>(j->x0.data()), reinterpret_cast<T *>(j->x1.data())};
+            const T *b = static_cast<const T *>(rhs);
+            T *xa = static_cast<T *>(x);
+            if (!direct) {
+                copy_async(ctx, j->rhs.data(), rhs, bytes);
+                copy_async(ctx, own[0], x, bytes);
+                b = reinterpret_cast<const T *>(j->rhs.data());
+                xa = own[0];
             }
-            copy_async(ctx, x, xa, bytes);
+            for (int s = 0; s < j->sweeps; ++s) {
+                // the last sweep ends in x where it does not start there
+                T *xb = xa == own[0] ? own[1] : own[0];
+                if (direct && s + 1 == j->sweeps && xa != x) xb = static_cast<T *>(x);
+                jacobi_sweep(ctx, c, reinterpret_cast<const T *>(j->dinv.data()), b, xa, xb, static_cast<T>(j->weight),
+                             nullptr, nullptr, static_cast<const T *>(nullptr));
+                xa = xb;
+            }
+            copy_async(ctx, x, xa, bytes);  // (nothing where xa is x)
         };
-        if (j->value_type == TF_F64) run(double{});
-        else run(float{});
-        cuda_check(cudaStreamSynchronize(ctx->stream), "Jacobi apply");
-        check_faults(ctx);
+        if (j->value_type == TF_F64) run(double{}, j->banded64);
+        else run(float{}, j->banded32);
+        check_faults(ctx);  // (synchronises the stream)
     });
 }
 
