@@ -99,9 +99,10 @@ void spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y);
 template <class T, class I>
 void autotune_spmv(tf_ctx *ctx, const Csr<T, I> &a, const T *x, T *y, int *stages, int *ctas_per_sm, int *cap_pct,
                    int *rows_per_thread, float *ms);
-// autotune_spmv the first time an operator of a's shape and storage is set
-// up in the process; later setups reuse the cached shape
-// (THERMOFEM_B200_SLICED_SHAPE forces the timing, and with it that shape).
+// The launch shape of an operator that is set up: the one cached for its
+// shape and storage; else by rule (fewer than 262,144 rows) or by timing the
+// few shapes that win on larger ones, and cached
+// (THERMOFEM_B200_SLICED_SHAPE forces the full timing, and with it that shape).
 template <class T, class I, class V = T>
 void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y);
 // The storage the SpMV family streams for a under its cached shape: true

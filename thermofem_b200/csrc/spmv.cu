@@ -174,17 +174,40 @@ __global__ void restrict_kernel(int64_t nc, const int32_t *__restrict__ off, con
 // the zero-guess sweep that follows it: b[c] = sum of fine[m] over the
 // members of aggregate c (restrict_kernel's order), x[c] = w d[c] b[c]
 // (jacobi_zero_kernel's expression).
+//
+// Three dependent loads (aggregate, member, value); with early (the
+// hierarchy is not written by any kernel in flight) the first two and the
+// diagonal come before the dependency wait, overlapping the kernel before.
 template <class T>
 __global__ void restrict_jacobi_zero_kernel(int64_t nc, const int32_t *__restrict__ off,
                                             const int32_t *__restrict__ mem, const T *__restrict__ fine,
-                                            T *__restrict__ b, const T *__restrict__ dinv, T *__restrict__ x, T w) {
-    pdl_enter();
+                                            T *__restrict__ b, const T *__restrict__ dinv, T *__restrict__ x, T w,
+                                            int early) {
+    if (!early) pdl_enter();
     const int64_t c = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (c >= nc) return;
+    const bool live = c < nc;
+    int32_t j0 = 0, j1 = 0, m[4] = {0, 0, 0, 0};
+    T d = 0;
+    if (live) {
+        j0 = off[c];
+        j1 = off[c + 1];
+        d = dinv[c];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (j0 + u < j1) m[u] = mem[j0 + u];
+    }
+    if (early) pdl_enter();
+    if (!live) return;
+    T v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = j0 + u < j1 ? fine[m[u]] : T(0);
     T s = 0;
-    for (int32_t j = off[c]; j < off[c + 1]; ++j) s += fine[mem[j]];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (j0 + u < j1) s += v[u];
+    for (int32_t j = j0 + 4; j < j1; ++j) s += fine[mem[j]];
     b[c] = s;
-    x[c] = w * dinv[c] * s;
+    x[c] = w * d * s;
 }
 
 template <class I>
@@ -352,13 +375,22 @@ __global__ void band_fill_kernel(int64_t rows, int64_t nslices, const int32_t *_
     }
 }
 
+// (the first map entry before the dependency wait when early)
 template <class T>
 __global__ void prolong_kernel(int64_t nf, const int32_t *__restrict__ map, const T *__restrict__ coarse,
-                               T *__restrict__ fine) {
-    pdl_enter();
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < nf;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        fine[i] += coarse[map[i]];
+                               T *__restrict__ fine, int early) {
+    if (!early) pdl_enter();
+    int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    int32_t c = i < nf ? map[i] : 0;
+    if (early) pdl_enter();
+    while (i < nf) {
+        const int64_t next = i + step;
+        const int32_t nc = next < nf ? map[next] : 0;
+        fine[i] += coarse[c];
+        i = next;
+        c = nc;
+    }
 }
 
 // Deterministic block reduction of up to 4 sums (fixed tree order).
@@ -623,8 +655,11 @@ void autotune_spmv(tf_ctx *ctx, const Csr<T, I> &a, const T *x, T *y, int *stage
 
 template <class T, class I, class V>
 void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y) {
-    if (!std::getenv("THERMOFEM_B200_SLICED_SHAPE") && tile::tuned(ctx, a)) return;
-    tile::autotune(ctx, a, x, y, nullptr);
+    // (a forced shape is taken by the full tuner)
+    const bool forced = std::getenv("THERMOFEM_B200_SLICED_SHAPE") != nullptr;
+    if (!forced && tile::tuned(ctx, a)) return;
+    if (!forced && a.rows < tile::kTimedRows) tile::take_rule(ctx, a);
+    else tile::autotune(ctx, a, x, y, nullptr, !forced);
 }
 
 template <class T, class I, class V>
@@ -668,7 +703,7 @@ void restrict_jacobi_zero(tf_ctx *ctx, int64_t nc, const int32_t *off, const int
                           const T *dinv, T *x, T w) {
     if (!nc) return;
     launch_kernel(ctx, "restrict_jacobi_zero", restrict_jacobi_zero_kernel<T>, grid_for(nc), kBlock, 0, nc, off, mem,
-                  fine, b, dinv, x, w);
+                  fine, b, dinv, x, w, ctx->stable ? 1 : 0);
 }
 
 bool indices_out_of_range(tf_ctx *ctx, int64_t n, const int32_t *idx, int32_t limit) {
@@ -818,7 +853,9 @@ bool build_sliced(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out, boo
     // the aggregated levels (30-45 % padding), 25 for FP32, where it does not
     // (128^3 PCG, one B200: FP64 36.1-36.8 vs 37.9-38.5 ms with 50 vs 25;
     // mixed 30.6 vs 29.4-29.8 ms).
-    int pad_pct = sizeof(T) == 8 ? 50 : 25;
+    // Operators that the wide kernel serves (tile::kWideRows) take a copy
+    // whatever the type: their launches are bound by round trips, not bytes.
+    int pad_pct = a.rows < tile::kWideRows ? 100 : (sizeof(T) == 8 ? 50 : 25);
     if (const char *v = std::getenv("THERMOFEM_B200_SLICED_PAD")) pad_pct = std::atoi(v);
     auto fits = [&](int64_t n) { return n < INT32_MAX && (n <= a.nnz + a.nnz * pad_pct / 100 || n <= 4096); };
     DeviceBuffer<int32_t> entries(static_cast<size_t>(nslices) + 1);
@@ -898,7 +935,8 @@ void restrict_sum(tf_ctx *ctx, int64_t nc, const int32_t *off, const int32_t *me
 template <class T>
 void prolong_add(tf_ctx *ctx, int64_t nf, const int32_t *map, const T *coarse, T *fine) {
     if (!nf) return;
-    launch_kernel(ctx, "prolong", prolong_kernel<T>, stride_grid(ctx, nf), kBlock, 0, nf, map, coarse, fine);
+    launch_kernel(ctx, "prolong", prolong_kernel<T>, stride_grid(ctx, nf), kBlock, 0, nf, map, coarse, fine,
+                  ctx->stable ? 1 : 0);
 }
 
 template <class T>

@@ -1207,6 +1207,14 @@ struct PipeConfig {
     int sliced{0}, sliced_ctas{4}, prefetch{1}, sliced_stages{2}, sliced_group{1};
 };
 
+// PipeConfig::prefetch of the direct kernel for small operators: whole slices
+// of up to kWideEntries slots are loaded ahead of the dependency wait and all
+// their gathers are in flight at once, where 8 at a time take as many round
+// trips to L2 as the row has eighths (SMALLLEVELS).  It needs 100-150
+// registers, so it is taken where one CTA per SM holds the operator.
+constexpr int kWideSlices = 2, kWideEntries = 24;
+constexpr int64_t kWideRows = 65536;
+
 // Stage capacity (entries) of the staged sliced kernel for a's copy in
 // groups of R tiles: R times its largest tile, or 0 when a stage would
 // exceed 96 KB.
@@ -1485,6 +1493,14 @@ void launch_sliced(tf_ctx *ctx, const Csr<T, I, V> &a, const XS &xs, const Epi &
     };
     auto go = [&](auto cols) {
         using Cols = decltype(cols);
+        if constexpr (std::is_same_v<Cols, OffsetCols>) {
+            if (cfg.prefetch == kWideSlices) {
+                constexpr auto kernel = sliced_kernel<T, kWideEntries, false, XS, Epi, Cols, V>;
+                launch_kernel(ctx, name, kernel, grid(resident_ctas<kernel>(kThreads, 0)), kThreads, 0, a.rows, a.sp,
+                              a.sv, cols, a.perm, early, xs, epi);
+                return;
+            }
+        }
         if (cfg.prefetch)
             launch_kernel(ctx, name, sliced_kernel<T, 8, true, XS, Epi, Cols, V>,
                           grid(resident_ctas<sliced_kernel<T, 8, true, XS, Epi, Cols, V>>(kThreads, 0)), kThreads, 0,
@@ -1578,8 +1594,35 @@ inline bool tune_log() {
     return on;
 }
 
+// The shape a setup takes for operators of fewer than kTimedRows rows without
+// timing anything.  Over 488 tuned operators (levels of heat, convection-
+// diffusion, 2-D and unstructured problems, three hierarchy types) the tuner's
+// choices there come down to these: row tiles in two stages, three CTAs per
+// SM (1.02-1.05 of the best shape's time on average, at launches of 4-10 us
+// whose own timing scatters by as much); copies read directly, three CTAs;
+// FP32 values under FP64 vectors staged (sliced) or prefetched (banded).
+constexpr int64_t kTimedRows = 262144;
+template <class T, class I, class V>
+PipeConfig rule_config(const Csr<T, I, V> &a) {
+    PipeConfig c{2, 3, 125, 1};
+    constexpr bool same = std::is_same_v<T, V>;
+    if (a.sp && a.bd) {
+        c.sliced = 1;
+        c.prefetch = same ? 0 : 1;
+        c.sliced_ctas = 3;
+    } else if (a.sp && a.cd) {
+        const bool wide = a.rows < kWideRows;
+        c.sliced = same || wide ? 1 : 2;
+        c.prefetch = wide ? kWideSlices : 0;
+        c.sliced_ctas = same || wide ? 3 : 2;
+    }
+    return c;
+}
+
+// quick: the shapes that win on larger operators only, fewer launches each
+// (setups); else every feasible shape (tf_autotune_spmv).
 template <class T, class I, class C, class V>
-PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y, float *best_ms) {
+PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y, float *best_ms, bool quick) {
     PipeConfig best{};
     float best_t = 0;
     cudaEvent_t e0, e1;
@@ -1595,19 +1638,20 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
                       static_cast<double>(kTuneFlushBytes) / 3;
     // (the context's second scratch arena: allocated once, kept for later setups)
     unsigned char *flush = cold ? static_cast<unsigned char *>(ctx->arena(kTuneFlushBytes, 1)) : nullptr;
+    const int warm = quick ? 1 : 2, reps = quick ? 3 : 5;
     auto time_cfg = [&](const PipeConfig &cfg) {
-        for (int w = 0; w < 2; ++w) launch(ctx, a, PlainX<T>{x}, TuneStore<T>{x, y, nullptr}, "autotune", &cfg);
+        for (int w = 0; w < warm; ++w) launch(ctx, a, PlainX<T>{x}, TuneStore<T>{x, y, nullptr}, "autotune", &cfg);
         if (!cold) {
             cuda_check(cudaEventRecord(e0, ctx->stream), "event");
-            for (int r = 0; r < 5; ++r) launch(ctx, a, PlainX<T>{x}, TuneStore<T>{x, y, nullptr}, "autotune", &cfg);
+            for (int r = 0; r < reps; ++r) launch(ctx, a, PlainX<T>{x}, TuneStore<T>{x, y, nullptr}, "autotune", &cfg);
             cuda_check(cudaEventRecord(e1, ctx->stream), "event");
             cuda_check(cudaEventSynchronize(e1), "event");
             float ms = 0;
             cuda_check(cudaEventElapsedTime(&ms, e0, e1), "event");
-            return ms / 5;
+            return ms / reps;
         }
         float total = 0;
-        for (int r = 0; r < 5; ++r) {
+        for (int r = 0; r < reps; ++r) {
             cuda_check(cudaMemsetAsync(flush, r, kTuneFlushBytes, ctx->stream), "tune flush");
             cuda_check(cudaMemcpyAsync(y, x, static_cast<size_t>(a.rows) * sizeof(T), cudaMemcpyDeviceToDevice,
                                        ctx->stream),
@@ -1620,48 +1664,51 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
             cuda_check(cudaEventElapsedTime(&ms, e0, e1), "event");
             total += ms;
         }
-        return total / 5;
+        return total / reps;
     };
     bool first = true;
-    for (int rpt : {1, 2}) {
-        for (int stages : {2, 3}) {
-            for (int ctas : {1, 2, 3, 4, 5, 6}) {
-                for (int pct : {100, 125}) {
-                    const PipeConfig cfg{stages, ctas, pct, rpt};
-                    const PipeShape p = pipe_shape<V, I, C>(a.rows, a.nnz, ctx->sm_count, cfg);
-                    if (p.smem * ctas > 220 * 1024) continue;
-                    if ((rpt == 1 && ctas < 2) || (rpt == 2 && ctas > 3)) continue;
-                    int resident = 0;
-                    if (rpt == 2) {
-                        allow_smem<csr_pipe_kernel<T, I, C, 2, PlainX<T>, TuneStore<T>, V>>(p.smem);
-                        resident = resident_ctas<csr_pipe_kernel<T, I, C, 2, PlainX<T>, TuneStore<T>, V>>(kThreads + 32,
-                                                                                                       p.smem);
-                    } else {
-                        allow_smem<csr_pipe_kernel<T, I, C, 1, PlainX<T>, TuneStore<T>, V>>(p.smem);
-                        resident = resident_ctas<csr_pipe_kernel<T, I, C, 1, PlainX<T>, TuneStore<T>, V>>(kThreads + 32,
-                                                                                                       p.smem);
-                    }
-                    if (resident < ctas) continue;
-                    const float ms = time_cfg(cfg);
-                    if (tune_log())
-                        std::fprintf(stderr,
-                                     "tf_autotune_spmv rows=%lld nnz=%lld T=%d C=%d rpt=%d stages=%d ctas=%d cap=%d%% "
-                                     "%.2f us\n",
-                                     static_cast<long long>(a.rows), static_cast<long long>(a.nnz),
-                                     static_cast<int>(sizeof(T)), static_cast<int>(sizeof(C)), rpt, stages, ctas, pct,
-                                     ms * 1e3f);
-                    if (first || ms < best_t) {
-                        best_t = ms;
-                        best = cfg;
-                        first = false;
-                    }
-                }
-            }
+    // row tiles
+    std::vector<PipeConfig> tiles;
+    const bool copied = std::is_same_v<I, int32_t> && a.sp && (a.bd || std::is_same_v<C, int16_t>);
+    if (quick) {
+        best = PipeConfig{2, 3, 125, 1};
+        // (an operator with a copy streams that)
+        if (!copied) tiles = {{2, 3, 125, 1}, {2, 4, 100, 1}, {2, 4, 125, 1}, {3, 2, 125, 1}, {2, 3, 100, 2}};
+    } else {
+        for (int rpt : {1, 2})
+            for (int stages : {2, 3})
+                for (int ctas : {1, 2, 3, 4, 5, 6})
+                    for (int pct : {100, 125})
+                        if (rpt == 1 ? ctas >= 2 : ctas <= 3) tiles.push_back({stages, ctas, pct, rpt});
+    }
+    for (const PipeConfig &cfg : tiles) {
+        const PipeShape p = pipe_shape<V, I, C>(a.rows, a.nnz, ctx->sm_count, cfg);
+        if (p.smem * cfg.ctas_per_sm > 220 * 1024) continue;
+        int resident = 0;
+        if (cfg.rpt == 2) {
+            allow_smem<csr_pipe_kernel<T, I, C, 2, PlainX<T>, TuneStore<T>, V>>(p.smem);
+            resident = resident_ctas<csr_pipe_kernel<T, I, C, 2, PlainX<T>, TuneStore<T>, V>>(kThreads + 32, p.smem);
+        } else {
+            allow_smem<csr_pipe_kernel<T, I, C, 1, PlainX<T>, TuneStore<T>, V>>(p.smem);
+            resident = resident_ctas<csr_pipe_kernel<T, I, C, 1, PlainX<T>, TuneStore<T>, V>>(kThreads + 32, p.smem);
+        }
+        if (resident < cfg.ctas_per_sm) continue;
+        const float ms = time_cfg(cfg);
+        if (tune_log())
+            std::fprintf(stderr,
+                         "tf_autotune_spmv rows=%lld nnz=%lld T=%d C=%d rpt=%d stages=%d ctas=%d cap=%d%% "
+                         "%.2f us\n",
+                         static_cast<long long>(a.rows), static_cast<long long>(a.nnz), static_cast<int>(sizeof(T)),
+                         static_cast<int>(sizeof(C)), cfg.rpt, cfg.stages, cfg.ctas_per_sm, cfg.cap_pct, ms * 1e3f);
+        if (first || ms < best_t) {
+            best_t = ms;
+            best = cfg;
+            first = false;
         }
     }
     if constexpr (std::is_same_v<I, int32_t>) {
         // a sliced copy (2-byte offsets: tuned under C = int16_t) or a banded one
-        if (a.sp && (a.bd || std::is_same_v<C, int16_t>)) {
+        if (copied) {
             // The sliced copy: next-tile prefetch on/off x resident CTAs per
             // SM, unless THERMOFEM_B200_SLICED_SHAPE="prefetch,ctas" forces one.
             int forced_pf = -1, forced_ctas = 0;
@@ -1687,6 +1734,19 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
                                         a3 < 1 ? 1 : a3, group);
                 else
                     shapes.emplace_back(1, forced_pf ? 1 : 0, forced_ctas < 1 ? 1 : forced_ctas, 1);
+            } else if (quick) {
+                const bool same = std::is_same_v<T, V>;
+                if (!a.bd) shapes = {{1, 0, 3, 1}, {1, 1, 3, 1}};
+                else if (!same) shapes = {{1, 1, 5, 1}, {1, 0, 5, 1}};
+                else if (sizeof(T) == 8) shapes = {{1, 0, 3, 1}, {1, 1, 3, 1}};
+                else shapes = {{1, 0, 4, 1}};
+                if (sliced_stage_cap(a, 1) && sizeof(T) == 8)
+                    shapes.emplace_back(2, 2, a.bd && same ? 4 : 2, 1);
+                if (a.bd && sizeof(T) == 8 && sliced_stage_cap(a, 2)) shapes.emplace_back(2, 2, 3, 2);
+                if (a.bd && sizeof(T) == 4 && sliced_stage_cap(a, 4)) {
+                    shapes.emplace_back(3, 2, 3, 4);
+                    shapes.emplace_back(3, 2, 2, 4);
+                }
             } else {
                 for (int pf : {0, 1})
                     for (int ctas : {2, 3, 4, 5, 6}) shapes.emplace_back(1, pf, ctas, 1);
@@ -1744,7 +1804,7 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
                     }
                 }
             }
-            if (!sfirst && (forced_pf >= 0 || sbest_t < best_t)) {
+            if (!sfirst && (forced_pf >= 0 || first || sbest_t < best_t)) {
                 best = sbest;
                 best_t = sbest_t;
             }
@@ -1763,11 +1823,20 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
 // CUDA events on the context stream) and caches the fastest for every later
 // launch over an operator of the same shape and storage.  y is overwritten.
 template <class T, class I, class V>
-PipeConfig autotune(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y, float *best_ms) {
+PipeConfig autotune(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y, float *best_ms, bool quick = false) {
     if (a.rows == 0 || !aligned16(a.rp) || (a.nnz && (!aligned16(a.ci) || !aligned16(a.val)))) return PipeConfig{};
     return with_columns(a, [&](auto cols) {
         using C = std::remove_cv_t<std::remove_pointer_t<decltype(cols)>>;
-        return autotune_columns<T, I, C, V>(ctx, a, x, y, best_ms);
+        return autotune_columns<T, I, C, V>(ctx, a, x, y, best_ms, quick);
+    });
+}
+
+// Caches the shape of rule_config for operators of a's shape and storage.
+template <class T, class I, class V>
+void take_rule(tf_ctx *ctx, const Csr<T, I, V> &a) {
+    with_columns(a, [&](auto cols) {
+        using C = std::remove_cv_t<std::remove_pointer_t<decltype(cols)>>;
+        store_config<T, I, C, V>(a.rows, a.nnz, ctx->sm_count, rule_config(a));
     });
 }
 
