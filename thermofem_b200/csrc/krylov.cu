@@ -22,7 +22,7 @@ namespace {
 enum : int { kRunning = -1 };
 
 struct KState {
-    double normB, tol, res, rho, rho_prev, alpha, omega, beta, curv;
+    double normB, tol, res, res0, rho, rho_prev, alpha, omega, beta, curv;
     int it, status, running, fresh, pmode, refresh, early, normal, copy_shadow, max_it, interval;
     unsigned tickets[8];  // last-CTA tickets of the reductions (zero between launches)
 };
@@ -64,6 +64,35 @@ __device__ __forceinline__ void sum_partials(const double *part, int parts, doub
     tile::block_reduce<K>(v);
 }
 
+// Calls use(i, load(i)) for the thread's positions i of a grid-stride walk
+// over [0, n), in their order, with the loads of kAhead of them in flight.
+// A reduction over fewer than kAheadRows rows has a fixed partition of at
+// most 512 CTAs whose threads take eight positions each: bound by eight round
+// trips to L2 when taken one after another, by one with all in flight
+// (AHEAD).  Longer vectors fill the GPU with the loads of more threads.
+constexpr int64_t kAheadRows = int64_t(1) << 20;
+template <int kAhead, class Load, class Use>
+__device__ __forceinline__ void walk(int64_t n, const Load &load, const Use &use) {
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i0 = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i0 < n; i0 += kAhead * step) {
+        decltype(load(i0)) t[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (i0 + u * step < n) t[u] = load(i0 + u * step);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (i0 + u * step < n) use(i0 + u * step, t[u]);
+    }
+}
+template <class T>
+struct Two {
+    T a, b;
+};
+template <class T>
+struct Four {
+    T a, b, c, d;
+};
+
 __device__ __forceinline__ void stop(KState *s, int status) {
     s->status = status;
     s->running = 0;
@@ -81,7 +110,7 @@ __global__ void k_init(KState *s, const double *pb, int nb, const double *pr, in
     if (threadIdx.x) return;
     s->normB = sqrt(vb[0]);
     s->tol = fmax(s->tol, s->res * s->normB);  // s->res carries rtol in, tol carries atol in
-    s->res = sqrt(vr[0]);
+    s->res = s->res0 = sqrt(vr[0]);
     s->it = 0;
     s->fresh = 1;
     s->refresh = s->early = s->copy_shadow = 0;
@@ -129,20 +158,33 @@ __global__ void k_reset(KState *s, KState init) {
     *s = init;
 }
 
-// Re-arms the WHILE node of the solve graph: one more iteration while the
+// Re-arms the WHILE nodes of the solve graph.  many: another round of
+// `unroll` iterations, while at least that many are to be expected at the
+// solve's own rate so far (an iteration after the end of the solve changes
+// nothing, but costs its kernels); one: one more iteration, while the
 // recurrence is running and below the iteration limit.
-__global__ void k_set_continue(cudaGraphConditionalHandle handle, const KState *s) {
+__global__ void k_set_continue(cudaGraphConditionalHandle many, cudaGraphConditionalHandle one, int unroll,
+                               const KState *s) {
     pdl_enter();
-    cudaGraphSetConditional(handle, (s->running && s->it < s->max_it) ? 1u : 0u);
+    const bool on = s->running && s->it < s->max_it;
+    if (unroll > 1) {
+        bool more = on && s->it + unroll <= s->max_it;
+        if (more && s->it > 0 && s->res < s->res0 && s->tol > 0) {
+            const float left = logf(static_cast<float>(s->res / s->tol)) * static_cast<float>(s->it);
+            more = left >= static_cast<float>(unroll) * logf(static_cast<float>(s->res0 / s->res));
+        }
+        cudaGraphSetConditional(many, more ? 1u : 0u);
+    }
+    cudaGraphSetConditional(one, on ? 1u : 0u);
 }
 
-template <class T, class Fin = tile::NoFinal>
+template <class T, int kAhead = 1, class Fin = tile::NoFinal>
 __global__ void k_dot(int64_t n, const T *__restrict__ x, const T *__restrict__ y, double *part, Fin fin = {}) {
     pdl_enter();
     double v[1] = {0.0};
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        v[0] += static_cast<double>(x[i]) * static_cast<double>(y[i]);
+    walk<kAhead>(
+        n, [&](int64_t i) { return Two<T>{x[i], y[i]}; },
+        [&](int64_t, const Two<T> &t) { v[0] += static_cast<double>(t.a) * static_cast<double>(t.b); });
     tile::block_reduce<1>(v);
     if (threadIdx.x == 0) part[blockIdx.x] = v[0];
     tile::finish(fin, part, gridDim.x);
@@ -151,17 +193,17 @@ __global__ void k_dot(int64_t n, const T *__restrict__ x, const T *__restrict__ 
 // z = T(xs) (the preconditioner's output in its own storage) and
 // sum_i r_i z_i, in the grid and order of k_dot: the conversion that ends
 // the preconditioner fused into the dot that follows it (same bits).
-template <class T, class S, class Fin>
+template <class T, class S, int kAhead, class Fin>
 __global__ void k_dot_from(int64_t n, const T *__restrict__ r, const S *__restrict__ xs, T *__restrict__ z,
                            double *part, Fin fin) {
     pdl_enter();
     double v[1] = {0.0};
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const T zi = static_cast<T>(xs[i]);
-        if (z) z[i] = zi;  // (null: the next step reads xs itself)
-        v[0] += static_cast<double>(r[i]) * static_cast<double>(zi);
-    }
+    walk<kAhead>(
+        n, [&](int64_t i) { return Two<T>{static_cast<T>(xs[i]), r[i]}; },
+        [&](int64_t i, const Two<T> &t) {
+            if (z) z[i] = t.a;  // (null: the next step reads xs itself)
+            v[0] += static_cast<double>(t.b) * static_cast<double>(t.a);
+        });
     tile::block_reduce<1>(v);
     if (threadIdx.x == 0) part[blockIdx.x] = v[0];
     tile::finish(fin, part, gridDim.x);
@@ -335,20 +377,21 @@ __device__ void cg_curv_step(KState *s, const double *part, int parts) {
     s->alpha = alpha;
 }
 
-template <class T, class Fin>
+template <class T, int kAhead, class Fin>
 __global__ void cg_xr(const KState *s, int64_t n, const T *__restrict__ p, const T *__restrict__ ap, T *__restrict__ x,
                       T *__restrict__ r, double *part, Fin fin) {
     pdl_enter();
     if (!s->running) return;
     const T alpha = static_cast<T>(s->alpha);
     double v[1] = {0.0};
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        x[i] += alpha * p[i];
-        const T ri = r[i] - alpha * ap[i];
-        r[i] = ri;
-        v[0] += static_cast<double>(ri) * static_cast<double>(ri);
-    }
+    walk<kAhead>(
+        n, [&](int64_t i) { return Four<T>{x[i], p[i], r[i], ap[i]}; },
+        [&](int64_t i, const Four<T> &t) {
+            x[i] = t.a + alpha * t.b;
+            const T ri = t.c - alpha * t.d;
+            r[i] = ri;
+            v[0] += static_cast<double>(ri) * static_cast<double>(ri);
+        });
     tile::block_reduce<1>(v);
     if (threadIdx.x == 0) part[blockIdx.x] = v[0];
     tile::finish(fin, part, gridDim.x);
@@ -460,20 +503,21 @@ __device__ void bi_alpha_step(KState *s, const double *part, int parts) {
 }
 
 // s = r - alpha v, x += alpha phat, sum s_i^2.
-template <class T, class Fin>
+template <class T, int kAhead, class Fin>
 __global__ void bi_s(const KState *st, int64_t n, const T *__restrict__ r, const T *__restrict__ v,
                      const T *__restrict__ ph, T *__restrict__ sv, T *__restrict__ x, double *part, Fin fin) {
     pdl_enter();
     if (!st->running) return;
     const T alpha = static_cast<T>(st->alpha);
     double acc[1] = {0.0};
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const T si = r[i] - alpha * v[i];
-        sv[i] = si;
-        x[i] += alpha * ph[i];
-        acc[0] += static_cast<double>(si) * static_cast<double>(si);
-    }
+    walk<kAhead>(
+        n, [&](int64_t i) { return Four<T>{r[i], v[i], x[i], ph[i]}; },
+        [&](int64_t i, const Four<T> &t) {
+            const T si = t.a - alpha * t.b;
+            sv[i] = si;
+            x[i] = t.c + alpha * t.d;
+            acc[0] += static_cast<double>(si) * static_cast<double>(si);
+        });
     tile::block_reduce<1>(acc);
     if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
     tile::finish(fin, part, gridDim.x);
@@ -522,20 +566,21 @@ __device__ void bi_omega_step(KState *s, const double *part, int parts) {
 }
 
 // x += omega shat, r = s - omega t, sum r_i^2.
-template <class T, class Fin>
+template <class T, int kAhead, class Fin>
 __global__ void bi_xr(const KState *st, int64_t n, const T *__restrict__ sh, const T *__restrict__ sv,
                       const T *__restrict__ t, T *__restrict__ x, T *__restrict__ r, double *part, Fin fin) {
     pdl_enter();
     if (!st->running || !st->normal) return;
     const T omega = static_cast<T>(st->omega);
     double acc[1] = {0.0};
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        x[i] += omega * sh[i];
-        const T ri = sv[i] - omega * t[i];
-        r[i] = ri;
-        acc[0] += static_cast<double>(ri) * static_cast<double>(ri);
-    }
+    walk<kAhead>(
+        n, [&](int64_t i) { return Four<T>{x[i], sh[i], sv[i], t[i]}; },
+        [&](int64_t i, const Four<T> &q) {
+            x[i] = q.a + omega * q.b;
+            const T ri = q.c - omega * q.d;
+            r[i] = ri;
+            acc[0] += static_cast<double>(ri) * static_cast<double>(ri);
+        });
     tile::block_reduce<1>(acc);
     if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
     tile::finish(fin, part, gridDim.x);
@@ -825,48 +870,65 @@ class KrylovImpl final : public Krylov {
         launch_kernel(ctx, "k_finish", k_finish, 1, 1024, 0, state_.data(), part_.data(), tiles_);
     }
 
-    // One graph for the whole solve: prefix, then a conditional WHILE node
-    // whose body is one iteration (it re-arms the condition from the device
-    // state at its end), then the suffix.  Falls back to the host loop when
-    // the driver refuses any step.
     // Adds the whole solve to graph g as one independent branch: (with
-    // reset, a kernel that loads the initial state) prefix, a conditional
-    // WHILE node whose body is one iteration (it re-arms the condition from
-    // the device state at its end), suffix.  Throws when CUDA refuses a
-    // step; the caller ends any capture left open.
+    // reset, a kernel that loads the initial state) prefix, the iterations,
+    // suffix.  The iterations are a conditional WHILE node of one, which
+    // re-arms its condition from the device state; short ones come in a
+    // first node of kUnroll at a time, since a turn of a WHILE node takes
+    // 5.6 us on B200 (a kernel of a programmatic chain 0.85 us): 128^2 FP64 PCG,
+    // 16 launches an iteration, 2.97 -> 2.51 ms with eight positions in flight
+    // (walk).  Not in batches, whose other systems fill the gap and whose
+    // graph would take 1.7 ms longer to build (12 systems), nor above
+    // kUnrollLaunches, where the turn is under 5 % of the iteration.  Throws
+    // when CUDA refuses a step; the caller ends any capture left open.
+    static constexpr int kUnroll = 4, kUnrollLaunches = 32;
     void add_solve_nodes(tf_ctx *ctx, cudaGraph_t g, bool reset) {
         const int64_t before = ctx->launches;
-        cudaGraphConditionalHandle handle;
-        cuda_check(cudaGraphConditionalHandleCreate(&handle, g, 0, cudaGraphCondAssignDefault), "condition");
+        cudaGraphConditionalHandle many{}, one;
+        cuda_check(cudaGraphConditionalHandleCreate(&one, g, 0, cudaGraphCondAssignDefault), "condition");
+        cudaGraph_t out = nullptr;
+        int unroll = 1;
+        auto add_loop = [&](cudaGraphConditionalHandle handle, int iterations, cudaGraphNode_t *node) {
+            cudaGraphNodeParams cp = {};
+            cp.type = cudaGraphNodeTypeConditional;
+            cp.conditional.handle = handle;
+            cp.conditional.type = cudaGraphCondTypeWhile;
+            cp.conditional.size = 1;
+            cuda_check(cudaGraphAddNode(node, g, nullptr, 0, &cp), "while node");
+            const int64_t b0 = ctx->launches;
+            cuda_check(cudaStreamBeginCaptureToGraph(ctx->stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                     cudaStreamCaptureModeThreadLocal),
+                       "capture body");
+            for (int k = 0; k < iterations; ++k) enqueue_iteration(ctx);
+            launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, many, one, unroll, state_.data());
+            cuda_check(cudaStreamEndCapture(ctx->stream, &out), "capture body end");
+            return ctx->launches - b0;
+        };
+        cudaGraphNode_t loop, rounds = nullptr;
+        per_iteration_ = add_loop(one, 1, &loop);
+        if (!reset && per_iteration_ <= kUnrollLaunches) {
+            unroll = kUnroll;
+            cuda_check(cudaGraphConditionalHandleCreate(&many, g, 0, cudaGraphCondAssignDefault), "condition");
+            add_loop(many, unroll, &rounds);
+        }
+        const int64_t p0 = ctx->launches;
         cuda_check(cudaStreamBeginCaptureToGraph(ctx->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
                    "capture prefix");
         if (reset) launch_kernel(ctx, "k_reset", k_reset, 1, 1, 0, state_.data(), initial_state());
         enqueue_prefix(ctx);
-        launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, handle, state_.data());
+        launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, many, one, unroll, state_.data());
         cudaStreamCaptureStatus st;
         const cudaGraphNode_t *deps = nullptr;
         size_t ndeps = 0;
         cuda_check(cudaStreamGetCaptureInfo(ctx->stream, &st, nullptr, nullptr, &deps, &ndeps), "capture info");
-        std::vector<cudaGraphNode_t> last(deps, deps + ndeps);
-        cudaGraph_t out = nullptr;
+        const std::vector<cudaGraphNode_t> last(deps, deps + ndeps);
         cuda_check(cudaStreamEndCapture(ctx->stream, &out), "capture prefix end");
-        prefix_launches_ = ctx->launches - before;
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = handle;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t loop;
-        cuda_check(cudaGraphAddNode(&loop, g, last.data(), last.size(), &cp), "while node");
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        const int64_t b0 = ctx->launches;
-        cuda_check(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0,
-                                                 cudaStreamCaptureModeThreadLocal),
-                   "capture body");
-        enqueue_iteration(ctx);
-        launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, handle, state_.data());
-        cuda_check(cudaStreamEndCapture(ctx->stream, &out), "capture body end");
-        per_iteration_ = ctx->launches - b0;
+        prefix_launches_ = ctx->launches - p0;
+        for (cudaGraphNode_t from : last) {
+            cudaGraphNode_t to = rounds ? rounds : loop;
+            cuda_check(cudaGraphAddDependencies(g, &from, &to, 1), "loop order");
+        }
+        if (rounds) cuda_check(cudaGraphAddDependencies(g, &rounds, &loop, 1), "loop order");
         const int64_t s0 = ctx->launches;
         cuda_check(cudaStreamBeginCaptureToGraph(ctx->stream, g, &loop, nullptr, 1, cudaStreamCaptureModeThreadLocal),
                    "capture suffix");
@@ -944,36 +1006,43 @@ class KrylovImpl final : public Krylov {
     }
 
     void enqueue_iteration(tf_ctx *ctx) {
+        if (n_ < kAheadRows) enqueue_iteration<8>(ctx);
+        else enqueue_iteration<1>(ctx);
+    }
+    template <int kAhead>
+    void enqueue_iteration(tf_ctx *ctx) {
         KState *s = state_.data();
         double *part = part_.data();
         unsigned *tk = s->tickets;
         const unsigned pg = static_cast<unsigned>(parts_);
+        // updates without a reduction: a thread per row while that fits
+        const unsigned ug = kAhead > 1 ? grid_for(n_) : pg;
         if (kind_ == TF_SOLVER_CG) {
             if (fuse_outer()) {
                 // z = M^-1 r stays in the hierarchy's finest level (its
                 // storage): the dot and the direction update read it there
                 const void *zs = hier_->apply_open(ctx, static_cast<const T *>(r_.data()));
                 if (hier_->storage_type() == TF_F32) {
-                    launch_kernel(ctx, "dot_rho_from", k_dot_from<T, float, CgRho>, pg, 256, 0, n_, r_.data(),
+                    launch_kernel(ctx, "dot_rho_from", k_dot_from<T, float, kAhead, CgRho>, pg, 256, 0, n_, r_.data(),
                                   static_cast<const float *>(zs), static_cast<T *>(nullptr), part, CgRho{s, tk + 0});
-                    launch_kernel(ctx, "cg_p", cg_p<T, float>, pg, 256, 0, s, n_, static_cast<const float *>(zs),
+                    launch_kernel(ctx, "cg_p", cg_p<T, float>, ug, 256, 0, s, n_, static_cast<const float *>(zs),
                                   p_.data());
                 } else {
-                    launch_kernel(ctx, "dot_rho_from", k_dot_from<T, double, CgRho>, pg, 256, 0, n_, r_.data(),
+                    launch_kernel(ctx, "dot_rho_from", k_dot_from<T, double, kAhead, CgRho>, pg, 256, 0, n_, r_.data(),
                                   static_cast<const double *>(zs), static_cast<T *>(nullptr), part, CgRho{s, tk + 0});
-                    launch_kernel(ctx, "cg_p", cg_p<T, double>, pg, 256, 0, s, n_, static_cast<const double *>(zs),
+                    launch_kernel(ctx, "cg_p", cg_p<T, double>, ug, 256, 0, s, n_, static_cast<const double *>(zs),
                                   p_.data());
                 }
             } else {
                 precondition(ctx, r_.data(), z_.data());
-                launch_kernel(ctx, "dot_rho", k_dot<T, CgRho>, pg, 256, 0, n_, r_.data(), z_.data(), part,
+                launch_kernel(ctx, "dot_rho", k_dot<T, kAhead, CgRho>, pg, 256, 0, n_, r_.data(), z_.data(), part,
                               CgRho{s, tk + 0});
-                launch_kernel(ctx, "cg_p", cg_p<T>, pg, 256, 0, s, n_, z_.data(), p_.data());
+                launch_kernel(ctx, "cg_p", cg_p<T>, ug, 256, 0, s, n_, z_.data(), p_.data());
             }
             tile::launch(ctx, csr(), tile::PlainX<T>{p_.data()},
                          SpmvDot<T, CgCurv>{q_.data(), p_.data(), &s->running, part, CgCurv{s, tk + 1}},
                          "spmv_dot_curv");
-            launch_kernel(ctx, "cg_xr_res", cg_xr<T, CgRes>, pg, 256, 0, s, n_, p_.data(), q_.data(), x_.data(),
+            launch_kernel(ctx, "cg_xr_res", cg_xr<T, kAhead, CgRes>, pg, 256, 0, s, n_, p_.data(), q_.data(), x_.data(),
                           r_.data(), part, CgRes{s, tk + 2});
             tile::launch(ctx, csr(), tile::PlainX<T>{x_.data()},
                          ResidualNorm<T, CgRefresh>{rhs_.data(), r_.data(), &s->refresh, part, CgRefresh{s, tk + 3}},
@@ -981,9 +1050,9 @@ class KrylovImpl final : public Krylov {
             return;
         }
         // BiCGStab: v = q_, phat = z_
-        launch_kernel(ctx, "dot_rho", k_dot<T, BiRho>, pg, 256, 0, n_, shadow_.data(), r_.data(), part,
+        launch_kernel(ctx, "dot_rho", k_dot<T, kAhead, BiRho>, pg, 256, 0, n_, shadow_.data(), r_.data(), part,
                       BiRho{s, tk + 0});
-        launch_kernel(ctx, "bi_p", bi_p<T>, pg, 256, 0, s, n_, r_.data(), q_.data(), p_.data());
+        launch_kernel(ctx, "bi_p", bi_p<T>, ug, 256, 0, s, n_, r_.data(), q_.data(), p_.data());
         const SpmvDot<T, BiAlpha> alpha_epi{q_.data(), shadow_.data(), &s->running, part, BiAlpha{s, tk + 1}};
         if (fuse_outer())
             preconditioned_spmv(ctx, p_.data(), z_.data(), alpha_epi, "spmv_dot_alpha_from");
@@ -991,7 +1060,7 @@ class KrylovImpl final : public Krylov {
             precondition(ctx, p_.data(), z_.data());
             tile::launch(ctx, csr(), tile::PlainX<T>{z_.data()}, alpha_epi, "spmv_dot_alpha");
         }
-        launch_kernel(ctx, "bi_s_norm", bi_s<T, BiSnorm>, pg, 256, 0, s, n_, r_.data(), q_.data(), z_.data(),
+        launch_kernel(ctx, "bi_s_norm", bi_s<T, kAhead, BiSnorm>, pg, 256, 0, s, n_, r_.data(), q_.data(), z_.data(),
                       s_.data(), x_.data(), part, BiSnorm{s, tk + 2});
         tile::launch(ctx, csr(), tile::PlainX<T>{x_.data()},
                      ResidualNorm<T, BiEarly>{rhs_.data(), r_.data(), &s->early, part, BiEarly{s, tk + 3}},
@@ -1003,12 +1072,12 @@ class KrylovImpl final : public Krylov {
             precondition(ctx, s_.data(), sh_.data());
             tile::launch(ctx, csr(), tile::PlainX<T>{sh_.data()}, omega_epi, "spmv_dot2_omega");
         }
-        launch_kernel(ctx, "bi_xr_res", bi_xr<T, BiRes>, pg, 256, 0, s, n_, sh_.data(), s_.data(), t_.data(),
+        launch_kernel(ctx, "bi_xr_res", bi_xr<T, kAhead, BiRes>, pg, 256, 0, s, n_, sh_.data(), s_.data(), t_.data(),
                       x_.data(), r_.data(), part, BiRes{s, tk + 5});
         tile::launch(ctx, csr(), tile::PlainX<T>{x_.data()}, ResidualNorm<T>{rhs_.data(), r_.data(), &s->refresh, part},
                      "residual_norm");
         launch_kernel(ctx, "bi_end", bi_end, 1, 1024, 0, s, part, tiles_);
-        launch_kernel(ctx, "copy_if", k_copy_if<T>, pg, 256, 0, &s->copy_shadow, n_, r_.data(), shadow_.data());
+        launch_kernel(ctx, "copy_if", k_copy_if<T>, ug, 256, 0, &s->copy_shadow, n_, r_.data(), shadow_.data());
     }
 
     int kind_;
