@@ -24,6 +24,7 @@ enum : int { kRunning = -1 };
 struct KState {
     double normB, tol, res, res0, rho, rho_prev, alpha, omega, beta, curv;
     int it, status, running, fresh, pmode, refresh, early, normal, copy_shadow, max_it, interval;
+    int go;  // PCG: running, and no residual refresh pending
     unsigned tickets[8];  // last-CTA tickets of the reductions (zero between launches)
 };
 
@@ -96,6 +97,7 @@ struct Four {
 __device__ __forceinline__ void stop(KState *s, int status) {
     s->status = status;
     s->running = 0;
+    s->go = 0;
 }
 
 // ---- shared steps --------------------------------------------------------
@@ -123,6 +125,7 @@ __global__ void k_init(KState *s, const double *pb, int nb, const double *pr, in
     else {
         s->status = kRunning;
         s->running = 1;
+        s->go = 1;
         s->copy_shadow = bicg;  // BiCGStab: shadow = r
     }
 }
@@ -330,7 +333,7 @@ struct ResidualNorm {
 // ---- PCG -----------------------------------------------------------------
 
 __device__ void cg_rho_step(KState *s, const double *part, int parts) {
-    if (!s->running) return;
+    if (!s->go) return;
     double v[1];
     sum_partials<1>(part, parts, v);
     if (threadIdx.x) return;
@@ -353,7 +356,7 @@ __device__ void cg_rho_step(KState *s, const double *part, int parts) {
 template <class T, class S = T>
 __global__ void cg_p(const KState *s, int64_t n, const S *__restrict__ z, T *__restrict__ p) {
     pdl_enter();
-    if (!s->running) return;
+    if (!s->go) return;
     const int mode = s->pmode;
     const T beta = static_cast<T>(s->beta);
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
@@ -364,7 +367,7 @@ __global__ void cg_p(const KState *s, int64_t n, const S *__restrict__ z, T *__r
 }
 
 __device__ void cg_curv_step(KState *s, const double *part, int parts) {
-    if (!s->running) return;
+    if (!s->go) return;
     double v[1];
     sum_partials<1>(part, parts, v);
     if (threadIdx.x) return;
@@ -381,7 +384,7 @@ template <class T, int kAhead, class Fin>
 __global__ void cg_xr(const KState *s, int64_t n, const T *__restrict__ p, const T *__restrict__ ap, T *__restrict__ x,
                       T *__restrict__ r, double *part, Fin fin) {
     pdl_enter();
-    if (!s->running) return;
+    if (!s->go) return;
     const T alpha = static_cast<T>(s->alpha);
     double v[1] = {0.0};
     walk<kAhead>(
@@ -400,7 +403,7 @@ __global__ void cg_xr(const KState *s, int64_t n, const T *__restrict__ p, const
 // ||r|| check and refresh decision (Cg.cuh:170-178); without a refresh the
 // iteration closes here (Cg.cuh:185-189).
 __device__ void cg_res_step(KState *s, const double *part, int parts) {
-    if (!s->running) return;
+    if (!s->go) return;
     double v[1];
     sum_partials<1>(part, parts, v);
     if (threadIdx.x) return;
@@ -409,6 +412,7 @@ __device__ void cg_res_step(KState *s, const double *part, int parts) {
     if (!isfinite(res)) return stop(s, TF_NONFINITE);
     if (res <= s->tol || s->it % s->interval == 0) {
         s->refresh = 1;
+        s->go = 0;  // until the refresh has run
         return;
     }
     s->rho_prev = s->rho;
@@ -427,6 +431,7 @@ __device__ void cg_refresh_step(KState *s, const double *part, int parts) {
     s->res = res;
     if (!isfinite(res) || res <= s->tol) return stop(s, TF_MAX_ITERATIONS);
     s->fresh = 1;
+    s->go = 1;
     s->rho_prev = s->rho;
     if (s->it >= s->max_it) stop(s, TF_MAX_ITERATIONS);
 }
@@ -877,17 +882,18 @@ class KrylovImpl final : public Krylov {
     // first node of kUnroll at a time, since a turn of a WHILE node takes
     // 5.6 us on B200 (a kernel of a programmatic chain 0.85 us): 128^2 FP64 PCG,
     // 16 launches an iteration, 2.97 -> 2.51 ms with eight positions in flight
-    // (walk).  Not in batches, whose other systems fill the gap and whose
+    // (walk), and 4 % less with the gated refresh once per round.  Not in batches, whose other systems fill the gap and whose
     // graph would take 1.7 ms longer to build (12 systems), nor above
     // kUnrollLaunches, where the turn is under 5 % of the iteration.  Throws
     // when CUDA refuses a step; the caller ends any capture left open.
-    static constexpr int kUnroll = 4, kUnrollLaunches = 32;
+    static constexpr int kUnroll = 5, kUnrollLaunches = 32;
     void add_solve_nodes(tf_ctx *ctx, cudaGraph_t g, bool reset) {
         const int64_t before = ctx->launches;
         cudaGraphConditionalHandle many{}, one;
         cuda_check(cudaGraphConditionalHandleCreate(&one, g, 0, cudaGraphCondAssignDefault), "condition");
         cudaGraph_t out = nullptr;
         int unroll = 1;
+        bool deferred = false;
         auto add_loop = [&](cudaGraphConditionalHandle handle, int iterations, cudaGraphNode_t *node) {
             cudaGraphNodeParams cp = {};
             cp.type = cudaGraphNodeTypeConditional;
@@ -899,7 +905,7 @@ class KrylovImpl final : public Krylov {
             cuda_check(cudaStreamBeginCaptureToGraph(ctx->stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                                      cudaStreamCaptureModeThreadLocal),
                        "capture body");
-            for (int k = 0; k < iterations; ++k) enqueue_iteration(ctx);
+            for (int k = 1; k <= iterations; ++k) enqueue_iteration(ctx, k == iterations || !deferred);
             launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, many, one, unroll, state_.data());
             cuda_check(cudaStreamEndCapture(ctx->stream, &out), "capture body end");
             return ctx->launches - b0;
@@ -907,6 +913,9 @@ class KrylovImpl final : public Krylov {
         cudaGraphNode_t loop, rounds = nullptr;
         per_iteration_ = add_loop(one, 1, &loop);
         if (!reset && per_iteration_ <= kUnrollLaunches) {
+            // PCG with a refresh interval of whole rounds (50 by default): the
+            // refresh once per round, the iterations before it never due one
+            deferred = kind_ == TF_SOLVER_CG && opt_.residual_refresh_interval % kUnroll == 0;
             unroll = kUnroll;
             cuda_check(cudaGraphConditionalHandleCreate(&many, g, 0, cudaGraphCondAssignDefault), "condition");
             add_loop(many, unroll, &rounds);
@@ -1005,12 +1014,15 @@ class KrylovImpl final : public Krylov {
         }
     }
 
-    void enqueue_iteration(tf_ctx *ctx) {
-        if (n_ < kAheadRows) enqueue_iteration<8>(ctx);
-        else enqueue_iteration<1>(ctx);
+    // refresh (PCG): with the gated residual refresh at its end; iterations
+    // recorded without it are followed by one that has it, and pause (s->go)
+    // where one is due before that.
+    void enqueue_iteration(tf_ctx *ctx, bool refresh = true) {
+        if (n_ < kAheadRows) enqueue_iteration<8>(ctx, refresh);
+        else enqueue_iteration<1>(ctx, refresh);
     }
     template <int kAhead>
-    void enqueue_iteration(tf_ctx *ctx) {
+    void enqueue_iteration(tf_ctx *ctx, bool refresh) {
         KState *s = state_.data();
         double *part = part_.data();
         unsigned *tk = s->tickets;
@@ -1021,18 +1033,15 @@ class KrylovImpl final : public Krylov {
             if (fuse_outer()) {
                 // z = M^-1 r stays in the hierarchy's finest level (its
                 // storage): the dot and the direction update read it there
-                const void *zs = hier_->apply_open(ctx, static_cast<const T *>(r_.data()));
-                if (hier_->storage_type() == TF_F32) {
-                    launch_kernel(ctx, "dot_rho_from", k_dot_from<T, float, kAhead, CgRho>, pg, 256, 0, n_, r_.data(),
-                                  static_cast<const float *>(zs), static_cast<T *>(nullptr), part, CgRho{s, tk + 0});
-                    launch_kernel(ctx, "cg_p", cg_p<T, float>, ug, 256, 0, s, n_, static_cast<const float *>(zs),
-                                  p_.data());
-                } else {
-                    launch_kernel(ctx, "dot_rho_from", k_dot_from<T, double, kAhead, CgRho>, pg, 256, 0, n_, r_.data(),
-                                  static_cast<const double *>(zs), static_cast<T *>(nullptr), part, CgRho{s, tk + 0});
-                    launch_kernel(ctx, "cg_p", cg_p<T, double>, ug, 256, 0, s, n_, static_cast<const double *>(zs),
-                                  p_.data());
-                }
+                auto from = [&](auto zero) {
+                    using S = decltype(zero);
+                    const S *zs = static_cast<const S *>(hier_->apply_open(ctx, static_cast<const T *>(r_.data())));
+                    launch_kernel(ctx, "dot_rho_from", k_dot_from<T, S, kAhead, CgRho>, pg, 256, 0, n_, r_.data(), zs,
+                                  static_cast<T *>(nullptr), part, CgRho{s, tk + 0});
+                    launch_kernel(ctx, "cg_p", cg_p<T, S>, ug, 256, 0, s, n_, zs, p_.data());
+                };
+                if (hier_->storage_type() == TF_F32) from(float{});
+                else from(double{});
             } else {
                 precondition(ctx, r_.data(), z_.data());
                 launch_kernel(ctx, "dot_rho", k_dot<T, kAhead, CgRho>, pg, 256, 0, n_, r_.data(), z_.data(), part,
@@ -1040,10 +1049,10 @@ class KrylovImpl final : public Krylov {
                 launch_kernel(ctx, "cg_p", cg_p<T>, ug, 256, 0, s, n_, z_.data(), p_.data());
             }
             tile::launch(ctx, csr(), tile::PlainX<T>{p_.data()},
-                         SpmvDot<T, CgCurv>{q_.data(), p_.data(), &s->running, part, CgCurv{s, tk + 1}},
-                         "spmv_dot_curv");
-            launch_kernel(ctx, "cg_xr_res", cg_xr<T, kAhead, CgRes>, pg, 256, 0, s, n_, p_.data(), q_.data(), x_.data(),
-                          r_.data(), part, CgRes{s, tk + 2});
+                         SpmvDot<T, CgCurv>{q_.data(), p_.data(), &s->go, part, CgCurv{s, tk + 1}}, "spmv_dot_curv");
+            launch_kernel(ctx, "cg_xr_res", cg_xr<T, kAhead, CgRes>, pg, 256, 0, s, n_, p_.data(), q_.data(),
+                          x_.data(), r_.data(), part, CgRes{s, tk + 2});
+            if (!refresh) return;
             tile::launch(ctx, csr(), tile::PlainX<T>{x_.data()},
                          ResidualNorm<T, CgRefresh>{rhs_.data(), r_.data(), &s->refresh, part, CgRefresh{s, tk + 3}},
                          "residual_refresh");
