@@ -251,8 +251,6 @@ class HierarchyImpl final : public Hierarchy {
             marks.mark(ctx, kPhLevel);
             const auto nc = csr_of(*native);
             row_max.allocate(static_cast<size_t>(nc.rows));
-            if (!row_stats(ctx, nc, row_max.data()))
-                fail(TF_ERR_INVALID, "Native AMG: missing/zero diagonal, non-finite value or reciprocal in hierarchy");
             levels_.emplace_back();
             Level<S, V> &l = levels_.back();
             l.n = nc.rows;
@@ -260,18 +258,42 @@ class HierarchyImpl final : public Hierarchy {
             l.rp.allocate(static_cast<size_t>(l.n) + 1);
             l.ci.allocate(static_cast<size_t>(l.nnz));
             l.val.allocate(static_cast<size_t>(l.nnz));
-            copy_async(ctx, l.rp.data(), nc.rp, (l.n + 1) * sizeof(int32_t));
-            copy_async(ctx, l.ci.data(), nc.ci, l.nnz * sizeof(int32_t));
-            convert(ctx, l.nnz, nc.val, l.val.data());
             for (auto *b : {&l.dinv, &l.rhs, &l.x0, &l.x1, &l.r}) b->allocate(static_cast<size_t>(l.n));
+            if (delta_columns_enabled() && l.nnz > 0) l.cd.allocate(static_cast<size_t>(l.nnz));
+            // the arrays, their checks and the sizes of the copies: two
+            // passes, one read-back
+            struct Report {
+                CopyShapes shapes;
+                int flags;
+            };
+            TempBuffer<Report> report(ctx, 1);
+            const size_t nslices = (static_cast<size_t>(l.n) + 31) / 32;
+            const bool copies = sliced_enabled() && l.nnz > 0;
+            TempBuffer<int32_t> bands(ctx, copies ? nslices + 1 : 0), slices(ctx, copies ? nslices + 1 : 0);
+            memset_async(ctx, report.data(), 0, sizeof(Report));
+            level_arrays(ctx, nc,
+                         LevelArrays<S, V>{l.rp.data(), l.ci.data(), l.val.data(), l.dinv.data(), l.cd.data(),
+                                           row_max.data()},
+                         &report.data()->flags);
+            if (copies)
+                copy_shapes(ctx, l.n, l.rp.data(), l.ci.data(), banded_enabled() ? bands.data() : nullptr,
+                            slices.data(), &report.data()->shapes);
+            const Report found = read_scalar(ctx, report.data());
+            if (found.flags & kLevelInvalid)
+                fail(TF_ERR_INVALID, "Native AMG: missing/zero diagonal, non-finite value or reciprocal in hierarchy");
             // The diagonal must also invert in the iteration precision.
-            inverse_diagonal(ctx, l.csr(), l.dinv.data());
+            if (found.flags & kLevelDiagonal) fail(TF_ERR_INVALID, "Missing or invalid diagonal");
+            if (found.flags & kLevelWide) l.cd.release();
             // learned damping: dinv_i scaled by omega_i, sweeps with weight 1
             if constexpr (std::is_same_v<S, V>) {
                 if (cfg_.model) learned_damping(ctx, *cfg_.model, l.csr(), depth, l.dinv.data());
             }
             marks.mark(ctx, kPhColumns);
-            column_copies(ctx, l);
+            if (copies && !(banded_enabled() && build_banded(ctx, l.values(), found.shapes, bands.data(), l.sl)) &&
+                l.cd.data()) {
+                if (sorted_slices_enabled()) build_sliced(ctx, l.values(), l.sl, true);
+                else build_sliced(ctx, l.values(), found.shapes, slices.data(), l.sl);
+            }
             marks.mark(ctx, kPhTuning);
             tune_level(ctx, l);
             LevelStats st;

@@ -148,6 +148,18 @@ void inverse_diagonal(tf_ctx *ctx, const Csr<T, I, V> &a, T *dinv);
 template <class I>
 bool delta_columns(tf_ctx *ctx, int64_t rows, const I *rp, const I *ci, int16_t *cd);
 bool delta_columns_enabled();
+// What a sliced or banded copy of an operator would hold: padded entries in
+// all and of the largest 256-row tile; band_bad: rows unsorted or with
+// repeated columns (1), a slice of more than 32 slots (2).
+struct CopyShapes {
+    unsigned long long band_total, slice_total;
+    int band_tile, slice_tile, band_bad;
+};
+// Enqueues the counts of both copies: entries per 32-row slice ((rows + 31) /
+// 32 + 1 values, the last 0) into bands and slices (null: not wanted) and the
+// totals into shapes (device).
+void copy_shapes(tf_ctx *ctx, int64_t rows, const int32_t *rp, const int32_t *ci, int32_t *bands, int32_t *slices,
+                 CopyShapes *shapes);
 // Builds the sliced copy of a (which must carry its 2-byte column offsets
 // cd): slice width = its longest row.  When the rows in their own order
 // would pad by more than THERMOFEM_B200_SLICED_PAD percent of nnz (default
@@ -160,7 +172,11 @@ bool delta_columns_enabled();
 // int32.  THERMOFEM_B200_SLICED=0 turns the copy off (sliced_enabled() false).
 template <class T>
 bool build_sliced(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out, bool allow_sort);
+template <class T>
+bool build_sliced(tf_ctx *ctx, const Csr<T, int32_t> &a, const CopyShapes &shapes, const int32_t *slices,
+                  SlicedCopy<T> &out);
 bool sliced_enabled();
+bool sorted_slices_enabled();
 // A banded copy of a (slices of 32 rows whose entries share their column
 // offsets slot by slot, SlicedCopy::band) when every row is sorted without
 // repeated columns, no slice needs more than 32 slots and the padding stays
@@ -168,6 +184,9 @@ bool sliced_enabled();
 // out released) otherwise.  THERMOFEM_B200_BANDED=0 turns it off.
 template <class T>
 bool build_banded(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out);
+template <class T>
+bool build_banded(tf_ctx *ctx, const Csr<T, int32_t> &a, const CopyShapes &shapes, const int32_t *bands,
+                  SlicedCopy<T> &out);
 bool banded_enabled();
 // Self-check of the bounded device waits: a kernel whose wait nothing ends
 // gives up after `polls` polls and raises the context's fault word; throws

@@ -77,6 +77,71 @@ __global__ void strength_edges(int n, const int32_t *__restrict__ rp, const int3
     if (!keys) count[i] = pos;
 }
 
+// A level's arrays from its native operator in one pass: the structure and the
+// values in their storage V, the inverse diagonal in the iteration precision S
+// (inverse_diagonal's expression), columns as row offsets, the largest
+// |off-diagonal| of each row and the checks (row_stats, inverse_diagonal,
+// delta_columns).  kG lanes share a row.  Bytes bound it on the finest level
+// (read once: 12 B an entry, written 10-14 B); on the others its launch does,
+// which is why one pass and one read-back of the flags took the place of six
+// launches and three read-backs a level.  Whole setup, with the copies' sizes
+// from one pass (copy_shapes): 2.1M rows FP32 8.9 -> 7.8 ms, a graph of 60k
+// rows 6.4 -> 5.5 ms.
+template <int kG, class S, class V>
+__global__ void level_arrays_kernel(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                                    const double *__restrict__ a, LevelArrays<S, V> out, int *flags) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const int64_t i64 = t / kG;
+    const int lane = static_cast<int>(t % kG);
+    int found = 0;
+    if (i64 < n) {
+        const int i = static_cast<int>(i64);
+        const int32_t begin = rp[i], end = rp[i + 1];
+        if (lane == 0) {
+            out.rp[i] = begin;
+            if (i == n - 1) out.rp[n] = end;
+        }
+        double diag = 0, mx = 0;
+        S d = S(0);
+        for (int32_t j = begin + lane; j < end; j += kG) {
+            const double v = a[j];
+            const int c = ci[j];
+            const V stored = static_cast<V>(v);
+            out.ci[j] = c;
+            out.val[j] = stored;
+            if (!isfinite(v)) found |= kLevelInvalid;
+            if (c == i) {
+                diag = v;
+                d += stored;
+            } else {
+                mx = fmax(mx, fabs(v));
+            }
+            if (out.cd) {
+                const int o = c - i;
+                if (o < -32767 || o > 32767) found |= kLevelWide;
+                else out.cd[j] = static_cast<int16_t>(o);
+            }
+        }
+        // (one lane holds the diagonal, the others 0)
+        const unsigned group = (kG == 32 ? 0xffffffffu : ((1u << (kG & 31)) - 1u)) << ((threadIdx.x & 31) / kG * kG);
+#pragma unroll
+        for (int o = kG / 2; o > 0; o >>= 1) {
+            mx = fmax(mx, __shfl_xor_sync(group, mx, o));
+            diag += __shfl_xor_sync(group, diag, o);
+            d += __shfl_xor_sync(group, d, o);
+        }
+        if (lane == 0) {
+            if (diag == 0 || !isfinite(diag) || !isfinite(1.0 / diag)) found |= kLevelInvalid;
+            const S inv = S(1) / d;
+            if (!isfinite(d) || d == S(0) || !isfinite(inv)) found |= kLevelDiagonal;
+            out.dinv[i] = inv;
+            out.row_max[i] = mx;
+        }
+    }
+    found = __reduce_or_sync(0xffffffffu, found);
+    if ((threadIdx.x & 31) == 0 && (found & ~*flags)) atomicOr(flags, found);
+}
+
 // Strength weights on the operator's own pattern: w[j] is the weight of edge
 // (i, c), the larger of its two directions' (GpuAggregation.cu:339-390), and
 // 0 where neither is strong and on the diagonal.  Such a graph needs no
@@ -795,6 +860,23 @@ std::unique_ptr<tf_dcsr> strength_graph(tf_ctx *ctx, const Csr<double, int32_t> 
     }
     return compress(ctx, n, m, keys.data(), w.data(), bits, 1);
 }
+
+template <class S, class V>
+void level_arrays(tf_ctx *ctx, const Csr<double, int32_t> &a, const LevelArrays<S, V> &out, int *flags) {
+    const int n = static_cast<int>(a.rows);
+    with_row_lanes(a, [&](auto lanes) {
+        constexpr int kG = decltype(lanes)::value;
+        level_arrays_kernel<kG, S, V><<<grid_for(static_cast<int64_t>(n) * kG), kBlock, 0, ctx->stream>>>(
+            n, a.rp, a.ci, a.val, out, flags);
+    });
+    launched(ctx, "level_arrays");
+}
+template void level_arrays<float, float>(tf_ctx *, const Csr<double, int32_t> &, const LevelArrays<float, float> &,
+                                         int *);
+template void level_arrays<double, double>(tf_ctx *, const Csr<double, int32_t> &, const LevelArrays<double, double> &,
+                                           int *);
+template void level_arrays<double, float>(tf_ctx *, const Csr<double, int32_t> &, const LevelArrays<double, float> &,
+                                          int *);
 
 void strength_weights(tf_ctx *ctx, const Csr<double, int32_t> &a, const double *row_max, double theta, double *w,
                       int *flags) {

@@ -20,6 +20,23 @@ std::unique_ptr<tf_dcsr> canonicalize(tf_ctx *ctx, const Csr<double, int32_t> &a
 std::unique_ptr<tf_dcsr> strength_graph(tf_ctx *ctx, const Csr<double, int32_t> &a, const double *row_max, double theta);
 int match_pairs(tf_ctx *ctx, const Csr<double, int32_t> &g, int rounds, int32_t *map);
 std::unique_ptr<tf_dcsr> contract_graph(tf_ctx *ctx, const Csr<double, int32_t> &g, const int32_t *map, int count);
+// Where a level's arrays go: structure, stored values, inverse diagonal,
+// columns as row offsets (null: none wanted), largest |off-diagonal| per row.
+template <class S, class V>
+struct LevelArrays {
+    int32_t *rp, *ci;
+    V *val;
+    S *dinv;
+    int16_t *cd;
+    double *row_max;
+};
+// Flags (device, zeroed by the caller): a value, diagonal or its reciprocal is
+// not usable (row_stats); the diagonal does not invert in S; a column lies
+// further than 32,767 from its row.
+constexpr int kLevelInvalid = 1, kLevelDiagonal = 2, kLevelWide = 4;
+template <class S, class V>
+void level_arrays(tf_ctx *ctx, const Csr<double, int32_t> &a, const LevelArrays<S, V> &out, int *flags);
+
 // The strength graph on a's own pattern: w[j] the weight of entry j's edge,
 // 0 where it is weak.  *flags (device): bit 0 some edge is strong; bit 1 a
 // strong edge has no entry for its other direction, and strength_graph has to

@@ -312,37 +312,69 @@ __device__ __forceinline__ int band_next(int64_t p, int64_t e, const int32_t *__
     return p < e ? ci[p] - row : INT_MAX;
 }
 
-__global__ void band_width_kernel(int64_t rows, int64_t nslices, const int32_t *__restrict__ rp,
-                                  const int32_t *__restrict__ ci, int32_t *__restrict__ entries,
-                                  unsigned long long *total, int *bad) {
+// Slots of every slice of the banded copy and, for slices in row order,
+// entries of the sliced one, with their totals and largest 256-row tiles (a
+// block is a tile).  bands / slices null: not wanted.
+__global__ void __launch_bounds__(256) copy_shapes_kernel(int64_t rows, int64_t nslices,
+                                                          const int32_t *__restrict__ rp,
+                                                          const int32_t *__restrict__ ci, int32_t *__restrict__ bands,
+                                                          int32_t *__restrict__ slices, CopyShapes *shapes) {
     pdl_enter();
+    __shared__ int tile[2];
+    if (threadIdx.x < 2) tile[threadIdx.x] = 0;
+    __syncthreads();
     const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     const int64_t s = t >> 5;  // uniform across the warp
-    if (s >= nslices) return;
     const int lane = static_cast<int>(t & 31);
-    const int row = static_cast<int>(t);
-    int64_t p = 0, e = 0;
-    if (t < rows) {
-        p = rp[t];
-        e = rp[t + 1];
-        for (int64_t k = p + 1; k < e; ++k)
-            if (ci[k] <= ci[k - 1]) atomicOr(bad, 1);
-    }
-    int slots = 0;
-    for (;;) {
-        const int mine = band_next(p, e, ci, row);
-        int m = mine;
-        for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (m == INT_MAX) break;
-        if (mine == m) ++p;
-        if (++slots > kBandMaxSlots) {
-            if (lane == 0) atomicOr(bad, 2);
-            return;
+    if (s < nslices) {
+        const int row = static_cast<int>(t);
+        int64_t p = 0, e = 0;
+        if (t < rows) {
+            p = rp[t];
+            e = rp[t + 1];
+        }
+        if (slices) {
+            int64_t len = e - p;
+            for (int o = 16; o > 0; o >>= 1) len = max(len, static_cast<int64_t>(__shfl_xor_sync(0xffffffffu, len, o)));
+            if (lane == 0) {
+                const bool huge = len * 32 > INT32_MAX / 8;  // (then the copy is never built)
+                slices[s] = huge ? INT32_MAX : static_cast<int>(len * 32);
+                if (huge) atomicAdd(&shapes->slice_total, 1ull << 40);
+                else atomicAdd(&tile[1], static_cast<int>(len * 32));
+            }
+        }
+        // (one slice that has no bands is enough: the others need no count)
+        int known = bands && lane == 0 ? *const_cast<volatile int *>(&shapes->band_bad) : 0;
+        known = __shfl_sync(0xffffffffu, known, 0);
+        if (bands && !known) {
+            int bad = 0;
+            for (int64_t k = p + 1; k < e; ++k)
+                if (ci[k] <= ci[k - 1]) bad = 1;
+            int slots = 0;
+            for (;;) {
+                const int mine = band_next(p, e, ci, row);
+                const int m = __reduce_min_sync(0xffffffffu, mine);
+                if (m == INT_MAX) break;
+                if (mine == m) ++p;
+                if (++slots > kBandMaxSlots) {
+                    bad = 2;
+                    break;
+                }
+            }
+            bad = __reduce_or_sync(0xffffffffu, bad);
+            if (lane == 0) {
+                if (bad) atomicOr(&shapes->band_bad, bad);
+                bands[s] = slots * 32;
+                atomicAdd(&tile[0], slots * 32);
+            }
         }
     }
-    if (lane == 0) {
-        entries[s] = slots * 32;
-        atomicAdd(total, static_cast<unsigned long long>(slots) * 32ull);
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const int sum = tile[threadIdx.x];
+        int *most = threadIdx.x ? &shapes->slice_tile : &shapes->band_tile;
+        if (sum > *const_cast<volatile int *>(most)) atomicMax(most, sum);
+        atomicAdd(threadIdx.x ? &shapes->slice_total : &shapes->band_total, static_cast<unsigned long long>(sum));
     }
 }
 
@@ -815,7 +847,7 @@ bool sliced_enabled() {
     return !(v && v[0] == '0');
 }
 
-static bool sorted_slices_enabled() {
+bool sorted_slices_enabled() {
     const char *v = std::getenv("THERMOFEM_B200_SLICED");
     return v && std::strcmp(v, "sorted") == 0;
 }
@@ -842,11 +874,9 @@ __global__ void slice_tile_max_kernel(int64_t nslices, const int32_t *__restrict
     atomicMax(tile_max, static_cast<unsigned long long>(sp[s1] - sp[s0]));
 }
 
+// Largest padded entry count of a sliced copy.
 template <class T>
-bool build_sliced(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out, bool allow_sort) {
-    out.release();
-    if (!a.rows || !a.nnz || !a.cd) return false;
-    const int64_t nslices = (a.rows + 31) / 32;
+static bool slices_fit(const Csr<T, int32_t> &a, int64_t n) {
     // padding of at most THERMOFEM_B200_SLICED_PAD percent of nnz (tiny
     // operators excepted; int32 entry starts).  Default 50 for FP64 values,
     // where the row-tile kernel's per-row work outweighs the padded bytes on
@@ -857,57 +887,93 @@ bool build_sliced(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out, boo
     // whatever the type: their launches are bound by round trips, not bytes.
     int pad_pct = a.rows < tile::kWideRows ? 100 : (sizeof(T) == 8 ? 50 : 25);
     if (const char *v = std::getenv("THERMOFEM_B200_SLICED_PAD")) pad_pct = std::atoi(v);
-    auto fits = [&](int64_t n) { return n < INT32_MAX && (n <= a.nnz + a.nnz * pad_pct / 100 || n <= 4096); };
-    DeviceBuffer<int32_t> entries(static_cast<size_t>(nslices) + 1);
-    int64_t n = slice_entries(ctx, a.rows, nslices, a.rp, nullptr, entries.data());
-    if (!fits(n)) {
-        if (!allow_sort || !sorted_slices_enabled()) return false;
-        out.perm.allocate(static_cast<size_t>(a.rows));
-        launch_kernel(ctx, "slice_sort", slice_sort_kernel<int32_t>, grid_for(a.rows, 256), 256, 0, a.rows, a.rp,
-                      out.perm.data());
-        n = slice_entries(ctx, a.rows, nslices, a.rp, out.perm.data(), entries.data());
-        if (!fits(n)) {
-            out.release();
-            return false;
-        }
-    }
+    return n < INT32_MAX && (n <= a.nnz + a.nnz * pad_pct / 100 || n <= 4096);
+}
+
+// The slices' starts from their entry counts, and their entries.
+template <class T>
+static void fill_sliced(tf_ctx *ctx, const Csr<T, int32_t> &a, const int32_t *entries, int64_t n, SlicedCopy<T> &out) {
+    const int64_t nslices = (a.rows + 31) / 32;
     out.sp.allocate(static_cast<size_t>(nslices) + 1);
-    scan_exclusive(ctx, nslices + 1, entries.data(), out.sp.data());
+    scan_exclusive(ctx, nslices + 1, entries, out.sp.data());
     out.val.allocate(static_cast<size_t>(n));
     out.col.allocate(static_cast<size_t>(n));
     launch_kernel(ctx, "slice_fill", slice_fill_kernel<T, int32_t>, grid_for(nslices * 32), kBlock, 0, a.rows,
                   nslices, a.rp, a.val, a.cd, out.perm.data(), out.sp.data(), out.val.data(), out.col.data());
-    DeviceBuffer<unsigned long long> tmax(1);
+    out.entries = n;
+}
+
+template <class T>
+bool build_sliced(tf_ctx *ctx, const Csr<T, int32_t> &a, const CopyShapes &shapes, const int32_t *slices,
+                  SlicedCopy<T> &out) {
+    out.release();
+    const int64_t n = static_cast<int64_t>(shapes.slice_total);
+    if (!a.rows || !a.nnz || !a.cd || !slices_fit(a, n)) return false;
+    fill_sliced(ctx, a, slices, n, out);
+    out.tile_max = shapes.slice_tile;
+    return true;
+}
+template bool build_sliced<float>(tf_ctx *, const Csr<float, int32_t> &, const CopyShapes &, const int32_t *,
+                                  SlicedCopy<float> &);
+template bool build_sliced<double>(tf_ctx *, const Csr<double, int32_t> &, const CopyShapes &, const int32_t *,
+                                   SlicedCopy<double> &);
+
+template <class T>
+bool build_sliced(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out, bool allow_sort) {
+    out.release();
+    if (!a.rows || !a.nnz || !a.cd) return false;
+    const int64_t nslices = (a.rows + 31) / 32;
+    TempBuffer<int32_t> entries(ctx, static_cast<size_t>(nslices) + 1);
+    TempBuffer<CopyShapes> shapes(ctx, 1);
+    copy_shapes(ctx, a.rows, a.rp, a.ci, nullptr, entries.data(), shapes.data());
+    const CopyShapes in_order = read_scalar(ctx, shapes.data());
+    if (build_sliced(ctx, a, in_order, entries.data(), out)) return true;
+    if (!allow_sort || !sorted_slices_enabled()) return false;
+    out.perm.allocate(static_cast<size_t>(a.rows));
+    launch_kernel(ctx, "slice_sort", slice_sort_kernel<int32_t>, grid_for(a.rows, 256), 256, 0, a.rows, a.rp,
+                  out.perm.data());
+    const int64_t n = slice_entries(ctx, a.rows, nslices, a.rp, out.perm.data(), entries.data());
+    if (!slices_fit(a, n)) {
+        out.release();
+        return false;
+    }
+    fill_sliced(ctx, a, entries.data(), n, out);
+    TempBuffer<unsigned long long> tmax(ctx, 1);
     memset_async(ctx, tmax.data(), 0, sizeof(unsigned long long));
     launch_kernel(ctx, "slice_tile_max", slice_tile_max_kernel, grid_for((nslices + 7) / 8), kBlock, 0, nslices,
                   out.sp.data(), tmax.data());
     out.tile_max = static_cast<int64_t>(read_scalar(ctx, tmax.data()));
-    out.entries = n;
     return true;
 }
 template bool build_sliced<float>(tf_ctx *, const Csr<float, int32_t> &, SlicedCopy<float> &, bool);
 template bool build_sliced<double>(tf_ctx *, const Csr<double, int32_t> &, SlicedCopy<double> &, bool);
 
-template <class T>
-bool build_banded(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out) {
-    out.release();
-    if (!a.rows || !a.nnz || a.rows >= INT32_MAX) return false;
-    const int64_t nslices = (a.rows + 31) / 32;
+void copy_shapes(tf_ctx *ctx, int64_t rows, const int32_t *rp, const int32_t *ci, int32_t *bands, int32_t *slices,
+                 CopyShapes *shapes) {
+    const int64_t nslices = (rows + 31) / 32;
+    memset_async(ctx, shapes, 0, sizeof(CopyShapes));
+    for (int32_t *p : {bands, slices})
+        if (p) memset_async(ctx, p + nslices, 0, sizeof(int32_t));  // the scans' sentinel
+    launch_kernel(ctx, "copy_shapes", copy_shapes_kernel, grid_for(nslices * 32), kBlock, 0, rows, nslices, rp, ci,
+                  bands, slices, shapes);
+}
+
+// Padding of at most THERMOFEM_B200_BANDED_PAD percent of nnz (default 10).
+static bool band_fits(const CopyShapes &s, int64_t nnz) {
     int pad_pct = 10;
     if (const char *v = std::getenv("THERMOFEM_B200_BANDED_PAD")) pad_pct = std::atoi(v);
-    DeviceBuffer<int32_t> entries(static_cast<size_t>(nslices) + 1);
-    DeviceBuffer<unsigned long long> total(1);
-    int *bad = static_cast<int *>(ctx->arena(sizeof(int), 1));
-    memset_async(ctx, entries.data(), 0, (nslices + 1) * sizeof(int32_t));
-    memset_async(ctx, total.data(), 0, sizeof(unsigned long long));
-    memset_async(ctx, bad, 0, sizeof(int));
-    launch_kernel(ctx, "band_width", band_width_kernel, grid_for(nslices * 32), kBlock, 0, a.rows, nslices, a.rp,
-                  a.ci, entries.data(), total.data(), bad);
-    if (read_scalar(ctx, bad)) return false;
-    const int64_t n = static_cast<int64_t>(read_scalar(ctx, total.data()));
-    if (n >= INT32_MAX || n > a.nnz + a.nnz * pad_pct / 100) return false;
+    const int64_t n = static_cast<int64_t>(s.band_total);
+    return s.band_bad == 0 && n < INT32_MAX && n <= nnz + nnz * pad_pct / 100;
+}
+
+template <class T>
+bool build_banded(tf_ctx *ctx, const Csr<T, int32_t> &a, const CopyShapes &shapes, const int32_t *bands,
+                  SlicedCopy<T> &out) {
+    out.release();
+    if (!a.rows || !a.nnz || a.rows >= INT32_MAX || !band_fits(shapes, a.nnz)) return false;
+    const int64_t nslices = (a.rows + 31) / 32, n = static_cast<int64_t>(shapes.band_total);
     out.sp.allocate(static_cast<size_t>(nslices) + 1);
-    scan_exclusive(ctx, nslices + 1, entries.data(), out.sp.data());
+    scan_exclusive(ctx, nslices + 1, bands, out.sp.data());
     out.val.allocate(static_cast<size_t>(n));
     // an even number of slots: the staged kernel copies whole 16-byte pairs
     const int64_t slots = n / 32, slots_even = (slots + 1) & ~int64_t(1);
@@ -915,13 +981,23 @@ bool build_banded(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out) {
     if (slots_even > slots) memset_async(ctx, out.band.data() + slots, 0, sizeof(int2));
     launch_kernel(ctx, "band_fill", band_fill_kernel<T>, grid_for(nslices * 32), kBlock, 0, a.rows, nslices, a.rp,
                   a.ci, a.val, out.sp.data(), out.val.data(), out.band.data());
-    DeviceBuffer<unsigned long long> tmax(1);
-    memset_async(ctx, tmax.data(), 0, sizeof(unsigned long long));
-    launch_kernel(ctx, "slice_tile_max", slice_tile_max_kernel, grid_for((nslices + 7) / 8), kBlock, 0, nslices,
-                  out.sp.data(), tmax.data());
-    out.tile_max = static_cast<int64_t>(read_scalar(ctx, tmax.data()));
+    out.tile_max = shapes.band_tile;
     out.entries = n;
     return true;
+}
+template bool build_banded<float>(tf_ctx *, const Csr<float, int32_t> &, const CopyShapes &, const int32_t *,
+                                  SlicedCopy<float> &);
+template bool build_banded<double>(tf_ctx *, const Csr<double, int32_t> &, const CopyShapes &, const int32_t *,
+                                   SlicedCopy<double> &);
+
+template <class T>
+bool build_banded(tf_ctx *ctx, const Csr<T, int32_t> &a, SlicedCopy<T> &out) {
+    out.release();
+    if (!a.rows || !a.nnz || a.rows >= INT32_MAX) return false;
+    TempBuffer<int32_t> bands(ctx, static_cast<size_t>((a.rows + 31) / 32) + 1);
+    TempBuffer<CopyShapes> shapes(ctx, 1);
+    copy_shapes(ctx, a.rows, a.rp, a.ci, bands.data(), nullptr, shapes.data());
+    return build_banded(ctx, a, read_scalar(ctx, shapes.data()), bands.data(), out);
 }
 template bool build_banded<float>(tf_ctx *, const Csr<float, int32_t> &, SlicedCopy<float> &);
 template bool build_banded<double>(tf_ctx *, const Csr<double, int32_t> &, SlicedCopy<double> &);
