@@ -7,9 +7,13 @@
 // (aggregates, member order, histograms, coarse sparsity) are meant to be
 // bit-identical to it, which is why every stage keeps the reference's
 // snapshot semantics: proposals of a matching round are all written before
-// any are accepted, absorption reads the pre-round map and sizes, member
-// slots are re-sorted after the atomic fill.  Sorting, reduction and scans
-// are the project's own (sort.cu).
+// any are accepted, and absorption accepts from one snapshot of proposals.
+// Rows are handled by themselves wherever a stage allows it: strength weights
+// lie on the operator's own pattern, the Galerkin product merges the rows of an
+// aggregate, aggregates are numbered by scans (scan.cuh), and their members are
+// sorted in place (at most four).  The sort over all coordinates (sort.cu) is
+// left for unsymmetric strength graphs, merged rows of more than 512 entries
+// and operators that arrive unsorted.
 #include <algorithm>
 #include <climits>
 #include <type_traits>
@@ -228,23 +232,30 @@ __device__ __forceinline__ bool better(int v, double s, int c, double score, int
 }
 
 // The proposal of open vertex v (v < 0: none), its best unmatched neighbour,
-// by kG consecutive lanes of a full warp; valid in each of them.  Weights are
-// read first: only an edge that would win gathers its neighbour.
+// by kG consecutive lanes of a full warp; valid in each of them.  Two entries
+// of a lane are in flight; only an edge that would win asks whether its
+// neighbour is taken, and in the first round nobody is.
 template <int kG>
-__device__ __forceinline__ int propose(const Matching &m, int v, int lane) {
+__device__ __forceinline__ int propose(const Matching &m, int v, int lane, bool first) {
     int best = -1;
     double score = 0;
+    auto consider = [&](double s, int32_t column) {
+        if (!(s > 0) || s < score) return;
+        const int c = m.vs.of(column);
+        if (c == v || !better(v, s, c, score, best) || (!first && m.taken[c])) return;
+        best = c;
+        score = s;
+    };
     for (int part = 0; part < 2 && v >= 0; ++part) {
         const int row = m.vs.lo ? (part ? m.vs.hi[v] : m.vs.lo[v]) : (part ? -1 : v);
         if (row < 0) break;
         const int32_t end = m.rp[row + 1];
-        for (int32_t j = m.rp[row] + lane; j < end; j += kG) {
-            const double s = m.w[j];
-            if (!(s > 0) || s < score) continue;
-            const int c = m.vs.of(m.ci[j]);
-            if (c == v || !better(v, s, c, score, best) || m.taken[c]) continue;
-            best = c;
-            score = s;
+        for (int32_t j = m.rp[row] + lane; j < end; j += 2 * kG) {
+            const bool two = j + kG < end;
+            const double s0 = m.w[j], s1 = two ? m.w[j + kG] : 0.0;
+            const int c0 = m.ci[j], c1 = two ? m.ci[j + kG] : 0;
+            consider(s0, c0);
+            consider(s1, c1);
         }
     }
     __syncwarp();
@@ -262,8 +273,9 @@ __device__ __forceinline__ int propose(const Matching &m, int v, int lane) {
 
 // Proposals of one round, from one snapshot of the matching
 // (GpuAggregation.cu:402-431).  Bound: reading the rows of the open vertices.
-// 128^3, finest level (2.1M rows, ncu): eight rounds' proposals 277 us and
-// acceptances 137 us; visiting every vertex in every round took 980 us.
+// 128^3 (2.1M rows, ncu): all proposals of a setup 1,487 us, 1,795 us with one
+// entry of a lane in flight; the finest level's first eight rounds took 980 us
+// when they visited every vertex, now 246 us and 138 us of acceptances.
 template <int kG>
 __global__ void __launch_bounds__(kBlock) match_propose(const __grid_constant__ Matching m, int round) {
     const int n = m.size(round), lane = threadIdx.x & 31;
@@ -271,7 +283,7 @@ __global__ void __launch_bounds__(kBlock) match_propose(const __grid_constant__ 
     for (int64_t k0 = (blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x - lane) / kG; k0 < n; k0 += step) {
         const int64_t k = k0 + lane / kG;
         const int v = k < n ? m.at(round, static_cast<int>(k)) : -1;
-        const int p = propose<kG>(m, v, lane % kG);
+        const int p = propose<kG>(m, v, lane % kG, round == 0);
         if (v >= 0 && lane % kG == 0) m.proposal[v] = p;
     }
 }
@@ -796,7 +808,7 @@ __device__ void match_in_block(const Matching &m, int rounds) {
         for (int k0 = (threadIdx.x - lane) / kG; k0 < n; k0 += nt / kG) {
             const int k = k0 + lane / kG;
             const int v = k < n ? m.at(round, k) : -1;
-            const int p = propose<kG>(m, v, lane % kG);
+            const int p = propose<kG>(m, v, lane % kG, round == 0);
             if (v >= 0 && lane % kG == 0) m.proposal[v] = p;
         }
         __syncthreads();
