@@ -1,13 +1,14 @@
-// coarse_cycle.cu -- the small levels of an AMG cycle as one thread-block
-// cluster working out of distributed shared memory.
+// coarse_cycle.cu -- the small levels of an AMG cycle as one launch out of
+// shared memory: one CTA where they fit (region_kernel), else one thread-block
+// cluster (tail_kernel).
 //
 // Below a few ten thousand rows every level operation of the cycle is a few
 // microseconds of launch and memory latency for well under a microsecond of
 // work: each launched kernel chains three or four dependent global-memory
 // round trips (row offsets, columns, gathered values).  Here the host records
 // the level steps of the sub-cycle that starts at the first small level (the
-// same recursion as the large levels: Cycle.cuh:35-63) and one cluster of up
-// to 16 CTAs runs them.  Rows of every level (fewer than 65536) are split
+// same recursion as the large levels: Cycle.cuh:35-63) and one launch runs
+// them.  The cluster form has up to 16 CTAs: rows of every level (fewer than 65536) are split
 // into equal contiguous ranges, one per CTA; a row's owner is a multiply-high
 // by the range length's reciprocal (exact below 65536 rows).  At the start
 // each CTA bulk-copies (cp.async.bulk, one copy per array, issued by as many
@@ -28,12 +29,12 @@
 // inverse with the warp-strided FP64 sum; so the cycle's result is the same
 // to the bit.
 //
-// When every level of the region fits in one CTA's shared memory (about
-// 25,000 nonzeros in FP32), the region is that one CTA: gathers are plain
-// shared-memory loads and steps are separated by __syncthreads.  Measured on
-// B200, a 16-CTA cluster barrier costs about a microsecond and a distributed
-// shared-memory round trip about half of one, so the cluster form only pays
-// when the levels do not fit in one CTA.
+// When the levels below the root fit in one CTA's shared memory (and the
+// root's vectors), the region is that one CTA: gathers are plain shared-memory
+// loads and steps are separated by __syncthreads.  Measured on B200, a 16-CTA
+// cluster barrier costs about a microsecond and a distributed shared-memory
+// round trip about half of one, so the cluster form is taken only when the
+// levels do not fit in one CTA.  The one-CTA form has its own comment below.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -1,5 +1,5 @@
-// coarse_cycle.cuh -- the small levels of an AMG cycle as one thread-block
-// cluster working out of distributed shared memory.
+// coarse_cycle.cuh -- the small levels of an AMG cycle as one launch out of
+// shared memory: one CTA, or a thread-block cluster where they do not fit.
 #pragma once
 #include <memory>
 #include <vector>
