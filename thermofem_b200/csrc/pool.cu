@@ -18,8 +18,9 @@
 namespace tfb {
 namespace {
 
-// Free bytes kept between calls, per device: what the 128^3 setup needs
-// (1.6 GiB of transient buffers), 2 % of the device's memory.
+// Free bytes kept between calls, per device: 2 % of its memory.  (A hierarchy
+// set up twice reserves 1.5 GiB in all at 128^3 and 2.7 GiB at 192^3, itself
+// included.)
 constexpr uint64_t kPoolKeep = uint64_t(4) << 30;
 
 struct DevicePool {

@@ -706,6 +706,8 @@ __global__ void __launch_bounds__(kThreads) sliced_kernel(int64_t rows, const in
         T y[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) y[g] = h.c[g] != kColPad ? xr(h.c[g]) : T(0);
+        // operands of the epilogue that wait for others of its own
+        if constexpr (requires { epi.late(pre); }) epi.late(pre);
         T acc = T(0);
 #pragma unroll
         for (int g = 0; g < G; ++g) acc += h.v[g] * y[g];
