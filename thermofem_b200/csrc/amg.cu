@@ -12,8 +12,8 @@
 // the reference's clear/visit semantics, but every level step is a fused
 // kernel: a pre-smooth from a zero guess is x = w Dinv b (no SpMV), the
 // residual is one pass, and the first post-smooth sweep reads x + P e on the
-// fly instead of running a separate prolongation.  The whole cycle is
-// captured once into a CUDA graph and replayed on every apply.
+// fly instead of running a separate prolongation.  The cycle is captured into
+// a CUDA graph on its second application and replayed from then on.
 #include <algorithm>
 #include <cstring>
 #include <istream>
@@ -236,7 +236,8 @@ class HierarchyImpl final : public Hierarchy {
         fuse_ = f ? std::atoi(f) : 1;
     }
     ~HierarchyImpl() override {
-        if (exec_) cudaGraphExecDestroy(exec_);
+        for (const Recorded &g : recorded_)
+            if (g.exec) cudaGraphExecDestroy(g.exec);
         if (viewed_) wait_for_device();
     }
 
@@ -538,16 +539,35 @@ class HierarchyImpl final : public Hierarchy {
         *lu = factored_ ? lu_.data() : nullptr;
         *pivots = factored_ ? piv_.data() : nullptr;
     }
-    int64_t kernels_per_cycle() const override { return per_cycle_; }
 
   private:
     template <class T>
     void apply_t(tf_ctx *ctx, const T *rhs, T *x) {
         StableScope stable(ctx);  // level operators are read-only from here on
         Level<S, V> &f = levels_.front();
-        convert(ctx, f.n, rhs, f.rhs.data());
-        run_cycle(ctx);
-        convert(ctx, f.n, levels_.front().x(), x);
+        // The finest level's first and last step touch the caller's vectors,
+        // which change from call to call, so they stay outside the graph: the
+        // zero-guess sweep reads rhs, the last post-smoothing sweep writes x.
+        // Converting before and after the whole cycle moved the finest vectors
+        // twice more (160^3, FP32 under FP64: 331 -> 315 us).
+        const bool outer = fuse_ > 0 && cfg_.o.cycle != TF_CYCLE_F && cfg_.o.pre_sweeps > 0 && levels_.size() > 1;
+        f.cur = 0;
+        if (outer) jacobi_zero_convert(ctx, f.n, f.dinv.data(), rhs, f.rhs.data(), f.x(), w_);
+        else convert(ctx, f.n, rhs, f.rhs.data());
+        if (const S *in = run_cycle(ctx, outer)) {
+            if constexpr (std::is_same_v<S, T>) {
+                jacobi_sweep(ctx, f.csr(), f.dinv.data(), f.rhs.data(), in, x, w_, nullptr, nullptr,
+                             static_cast<const S *>(nullptr));
+                return;
+            } else if constexpr (std::is_same_v<S, float>) {
+                jacobi_sweep_widened(ctx, f.csr(), f.dinv.data(), f.rhs.data(), in, x, w_);
+                return;
+            } else {
+                jacobi_sweep(ctx, f.csr(), f.dinv.data(), f.rhs.data(), in, f.x(), w_, nullptr, nullptr,
+                             static_cast<const S *>(nullptr));
+            }
+        }
+        convert(ctx, f.n, f.x(), x);
     }
     const void *apply_open(tf_ctx *ctx, const double *rhs) override { return open_t(ctx, rhs); }
     const void *apply_open(tf_ctx *ctx, const float *rhs) override { return open_t(ctx, rhs); }
@@ -570,25 +590,44 @@ class HierarchyImpl final : public Hierarchy {
         return levels_.front().x();
     }
 
-    void run_cycle(tf_ctx *ctx) {
+    // The cycle; with outer set, without the finest level's zero-guess sweep
+    // (done before) and, where it ends in one, without its last sweep: the
+    // vector that sweep starts from is returned, else null.
+    const S *run_cycle(tf_ctx *ctx, bool outer = false) {
         cudaStreamCaptureStatus capturing;
         cuda_check(cudaStreamIsCapturing(ctx->stream, &capturing), "capture status");
         if (capturing != cudaStreamCaptureStatusNone) {  // inside a caller's capture: record inline
-            enqueue(ctx);
-            return;
+            enqueue(ctx, outer);
+            return last_in_;
         }
-        if (!exec_ && !capture_failed_) capture(ctx);
-        if (exec_) {
-            cuda_check(cudaGraphLaunch(exec_, ctx->stream), "cycle graph launch");
-            ctx->launches += per_cycle_;
-            for (size_t d = 0; d < levels_.size(); ++d) levels_[d].cur = final_cur_[d];
-            visits = captured_visits_;
-        } else {
-            enqueue(ctx);
+        // The first cycle is launched step by step: capturing and
+        // instantiating takes longer than it saves in one cycle (160^3: a new
+        // hierarchy's first application 806 -> 346 us).
+        Recorded &g = recorded_[outer];
+        if (!g.exec && !capture_failed_ && g.used) capture(ctx, g, outer);
+        g.used = true;
+        if (!g.exec) {
+            enqueue(ctx, outer);
+            return last_in_;
         }
+        cuda_check(cudaGraphLaunch(g.exec, ctx->stream), "cycle graph launch");
+        ctx->launches += g.launches;
+        for (size_t d = 0; d < levels_.size(); ++d) levels_[d].cur = g.cur[d];
+        visits = g.visits;
+        return g.last_in;
     }
 
-    void capture(tf_ctx *ctx) {
+    // A captured cycle, and the state it leaves.
+    struct Recorded {
+        cudaGraphExec_t exec{nullptr};
+        bool used{false};
+        int64_t launches{0};
+        std::vector<int> cur;
+        std::vector<int64_t> visits;
+        const S *last_in{nullptr};
+    };
+
+    void capture(tf_ctx *ctx, Recorded &g, bool outer) {
         if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
             capture_failed_ = true;
@@ -597,7 +636,7 @@ class HierarchyImpl final : public Hierarchy {
         const int64_t before = ctx->launches;
         cudaGraph_t graph = nullptr;
         try {
-            enqueue(ctx);
+            enqueue(ctx, outer);
         } catch (const Failure &) {
             // a step the driver cannot capture: run uncaptured from now on
             cudaStreamEndCapture(ctx->stream, &graph);
@@ -607,23 +646,26 @@ class HierarchyImpl final : public Hierarchy {
             capture_failed_ = true;
             return;
         }
-        per_cycle_ = ctx->launches - before;
+        g.launches = ctx->launches - before;
         ctx->launches = before;
         cuda_check(cudaStreamEndCapture(ctx->stream, &graph), "cycle capture");
-        cudaError_t e = cudaGraphInstantiate(&exec_, graph, 0);
+        cudaError_t e = cudaGraphInstantiate(&g.exec, graph, 0);
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) {
             cudaGetLastError();
-            exec_ = nullptr;
+            g.exec = nullptr;
             capture_failed_ = true;
             return;
         }
-        final_cur_.resize(levels_.size());
-        for (size_t d = 0; d < levels_.size(); ++d) final_cur_[d] = levels_[d].cur;
-        captured_visits_ = visits;
+        g.cur.clear();
+        for (const auto &l : levels_) g.cur.push_back(l.cur);
+        g.visits = visits;
+        g.last_in = last_in_;
     }
 
-    void enqueue(tf_ctx *ctx) {
+    void enqueue(tf_ctx *ctx, bool outer = false) {
+        outer_ = outer;
+        last_in_ = nullptr;
         for (auto &l : levels_) l.cur = 0;
         std::fill(visits.begin(), visits.end(), 0);
         entry_ = 0;
@@ -631,7 +673,12 @@ class HierarchyImpl final : public Hierarchy {
         pr_ = {};
         pw_ = {};
         cycle(ctx, cfg_.o.cycle, 0, true);
-        if (!dry_) flush(ctx);
+        if (dry_) return;
+        if (outer && pw_.kind == kWriteSweep && pw_.l == &levels_.front()) {
+            last_in_ = pw_.xin;
+            pw_ = {};
+        }
+        flush(ctx);
     }
 
     // ---- level operations: launched, or recorded as a small-level program step ----
@@ -657,6 +704,7 @@ class HierarchyImpl final : public Hierarchy {
             s.xout = l.x();
             rec_.push_back(s);
         } else if (!dry_) {
+            if (outer_ && &l == &levels_.front()) return;  // done before the cycle
             if (fusing() && pin_.src && &l == &levels_.front()) {
                 const PendingInput in = pin_;
                 pin_ = {};
@@ -1067,11 +1115,10 @@ class HierarchyImpl final : public Hierarchy {
     // a caller was given device pointers into the hierarchy, which it may be
     // reading on streams of its own
     mutable bool viewed_{false};
-    cudaGraphExec_t exec_{nullptr};
+    Recorded recorded_[2];  // the whole cycle; without the finest level's outer steps
     bool capture_failed_{false};
-    int64_t per_cycle_{0};
-    std::vector<int> final_cur_;
-    std::vector<int64_t> captured_visits_;
+    bool outer_{false};  // the cycle being enqueued leaves those to its caller
+    const S *last_in_{nullptr};
     // small-level sub-cycles (one cluster launch each)
     size_t coop_from_{~size_t(0)};
     bool recording_{false}, dry_{false};

@@ -59,8 +59,6 @@ class Hierarchy {
     // The coarse level's LU factor (rows x rows doubles, row-major, and the
     // pivot row of each step), rows = 0 when the coarse solve is Jacobi.
     virtual void coarse_factor(int *rows, const double **lu, const int32_t **pivots) const = 0;
-    // Kernels launched by one cycle (graph replay counts them too).
-    virtual int64_t kernels_per_cycle() const = 0;
     // Writes the hierarchy (restore_hierarchy reads it back).
     virtual void save(tf_ctx *ctx, std::ostream &out) const = 0;
 

@@ -119,6 +119,9 @@ void residual(tf_ctx *ctx, const Csr<T, I, V> &a, const T *b, const T *x, T *r);
 template <class T, class I, class V = T>
 void jacobi_sweep(tf_ctx *ctx, const Csr<T, I, V> &a, const T *dinv, const T *b, const T *x, T *xo, T w,
                   const float *row_w, const int32_t *map, const T *e);
+// The same without a map, its FP32 result stored in FP64.
+void jacobi_sweep_widened(tf_ctx *ctx, const Csr<float, int32_t> &a, const float *dinv, const float *b, const float *x,
+                          double *xo, float w);
 // xo = x + w Dinv (b - A x), and fine[mem[k]] += xo[c] for k in
 // [off[c], off[c+1]) (the prolongation of the result fused in).
 template <class T, class I, class V = T>

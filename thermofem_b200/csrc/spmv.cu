@@ -53,7 +53,8 @@ struct ResidualOut {
 
 // x_out = x~ + (w Dinv) (b - A x~), the reference's update expression
 // x += w * d * (b - a) (IterationContext.cu:26-32).
-template <class T>
+// O: the type it is stored in (FP64 for a caller of an FP32 cycle).
+template <class T, class O = T>
 struct JacobiOut {
     static constexpr int kReduce = 0;
     struct Pre {
@@ -61,7 +62,7 @@ struct JacobiOut {
     };
     const T *__restrict__ dinv;
     const T *__restrict__ b;
-    T *__restrict__ xo;
+    O *__restrict__ xo;
     const float *__restrict__ row_w;
     T w;
     double *partial{nullptr};
@@ -71,7 +72,7 @@ struct JacobiOut {
         return {xs(i), dinv[i], b[i], row_w ? static_cast<T>(row_w[i]) : w};
     }
     __device__ __forceinline__ void operator()(int64_t i, T acc, const Pre &p, double (&)[1]) const {
-        xo[i] = p.x + p.w * p.d * (p.b - acc);
+        xo[i] = static_cast<O>(p.x + p.w * p.d * (p.b - acc));
     }
 };
 
@@ -742,6 +743,12 @@ void jacobi_sweep(tf_ctx *ctx, const Csr<T, I, V> &a, const T *dinv, const T *b,
         launch_tile(ctx, a, ProlongX<T>{x, map, e}, epi, "jacobi_prolong");
     else
         launch_tile(ctx, a, PlainX<T>{x}, epi, "jacobi");
+}
+
+void jacobi_sweep_widened(tf_ctx *ctx, const Csr<float, int32_t> &a, const float *dinv, const float *b, const float *x,
+                          double *xo, float w) {
+    launch_tile(ctx, a, PlainX<float>{x}, JacobiOut<float, double>{dinv, b, xo, nullptr, w, nullptr},
+                "jacobi_widened");
 }
 
 template <class T, class I, class V>
