@@ -411,32 +411,35 @@ __device__ __forceinline__ unsigned group_mask() {
     return (kG == 32 ? 0xffffffffu : ((1u << (kG & 31)) - 1u)) << ((threadIdx.x & 31) / kG * kG);
 }
 
-// Row i by kG consecutive lanes.
+__device__ __forceinline__ bool proposes(const Absorption &a, int i) {
+    return a.sizes[a.map[i]] == 1;  // (nobody writes sizes while proposals are made)
+}
+
+// The proposal of singleton i by kG consecutive lanes.
 template <int kG>
 __device__ __forceinline__ void propose_absorption(const Absorption &a, int i, int lane) {
     const auto [rp, ci, w, count, map, sizes, slots, proposal, scores] = a;
     int best = -1;
     double score = 0;
-    if (sizes[map[i]] == 1) {  // (nobody writes sizes here: uniform over the group)
 #pragma unroll 2
-        for (int32_t j = rp[i] + lane; j < rp[i + 1]; j += kG) {
-            const double s = w[j];
-            if (s <= 0 || s < score) continue;
-            const int c = map[ci[j]];
-            if (sizes[c] < 2 || sizes[c] >= 4) continue;
-            if (s > score || (s == score && (best < 0 || c < best))) {
-                best = c;
-                score = s;
-            }
+    for (int32_t j = rp[i] + lane; j < rp[i + 1]; j += kG) {
+        const double s = w[j];
+        if (s <= 0 || s < score) continue;
+        const int c = map[ci[j]];
+        if (sizes[c] < 2 || sizes[c] >= 4) continue;
+        if (s > score || (s == score && (best < 0 || c < best))) {
+            best = c;
+            score = s;
         }
+    }
+    __syncwarp(group_mask<kG>());
 #pragma unroll
-        for (int o = kG / 2; o > 0; o >>= 1) {
-            const double s = __shfl_xor_sync(group_mask<kG>(), score, o);
-            const int c = __shfl_xor_sync(group_mask<kG>(), best, o);
-            if (c >= 0 && (s > score || (s == score && (best < 0 || c < best)))) {
-                best = c;
-                score = s;
-            }
+    for (int o = kG / 2; o > 0; o >>= 1) {
+        const double s = __shfl_xor_sync(group_mask<kG>(), score, o);
+        const int c = __shfl_xor_sync(group_mask<kG>(), best, o);
+        if (c >= 0 && (s > score || (s == score && (best < 0 || c < best)))) {
+            best = c;
+            score = s;
         }
     }
     if (lane == 0) {
@@ -455,12 +458,14 @@ __device__ __forceinline__ void propose_absorption(const Absorption &a, int i, i
 // Bound by the latency of one row after another: a lane per row and aggregate
 // (8 + 8 launches of a 60k-row graph setup) took 444 + 155 us, and that setup
 // 5.47 ms; lanes by the mean row length 4.93 ms.
+__device__ __forceinline__ bool accepts(const Absorption &a, int c) {
+    return c < *a.count && a.sizes[c] >= 2 && a.sizes[c] < 4;
+}
+
 template <int kG>
 __device__ __forceinline__ void accept_absorption(const Absorption &a, int c, int lane) {
     const auto [rp, ci, w, count, map, sizes, slots, proposal, scores] = a;
-    if (c >= *count) return;
     const int size = sizes[c];
-    if (size < 2 || size >= 4) return;
     int s0 = -1, s1 = -1;  // best and second proposer
     double w0 = -1, w1 = -1;
     auto offer = [&](int i, double s) {
@@ -502,15 +507,35 @@ __device__ __forceinline__ void accept_absorption(const Absorption &a, int c, in
     if (now != size) sizes[c] = now;
 }
 
+// One thread looks at each row; the singletons are listed per warp, and kG
+// lanes share one of the list: with kG lanes on every row most of them waited
+// on gathers for rows of other aggregates (heat operator of 2.1M rows, twelve
+// launches: 305 -> 162 us).  Whole warps (long rows) have no list, a warp
+// would go through it alone.  Aggregates with room are too many of all for a
+// list to pay (329 us without, 372 us with one).
 template <int kG>
-__global__ void propose_absorption_kernel(int n, const __grid_constant__ Absorption a) {
+__global__ void __launch_bounds__(kBlock) propose_absorption_kernel(int n, const __grid_constant__ Absorption a) {
+    constexpr int kLook = kG == 32 ? 32 : 1;  // lanes that look at a row
+    __shared__ int list[kBlock];
     const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (t / kG < n) propose_absorption<kG>(a, static_cast<int>(t / kG), static_cast<int>(t % kG));
+    const int i = static_cast<int>(t / kLook), lane = threadIdx.x & 31;
+    const bool mine = t / kLook < n && proposes(a, i);
+    if (t / kLook < n && !mine) a.proposal[i] = -1;
+    if constexpr (kG == 32) {
+        if (mine) propose_absorption<kG>(a, i, lane);
+    } else {
+        const unsigned all = __ballot_sync(0xffffffffu, mine);
+        int *of_warp = list + (threadIdx.x - lane);
+        if (mine) of_warp[__popc(all & ((1u << lane) - 1u))] = i;
+        __syncwarp();
+        for (int k = lane / kG; k < __popc(all); k += 32 / kG) propose_absorption<kG>(a, of_warp[k], lane % kG);
+    }
 }
 template <int kG>
-__global__ void accept_absorption_kernel(int n, const __grid_constant__ Absorption a) {
+__global__ void __launch_bounds__(kBlock) accept_absorption_kernel(int n, const __grid_constant__ Absorption a) {
     const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (t / kG < n) accept_absorption<kG>(a, static_cast<int>(t / kG), static_cast<int>(t % kG));
+    const int c = static_cast<int>(t / kG);
+    if (t / kG < n && accepts(a, c)) accept_absorption<kG>(a, c, static_cast<int>(t % kG));
 }
 
 // Scan input: the aggregate counted under its size, 1 to 4 rows (an emptied
@@ -835,9 +860,13 @@ __global__ void __launch_bounds__(scan_detail::kMidThreads, 1) aggregate_one_cta
     scan_in_block<1>(s.n + 1, s.to_aggregates.f, s.to_aggregates);
     for (int round = 0; s.absorb && round < 2; ++round) {
         const int lane = threadIdx.x % kG, groups = blockDim.x / kG;
-        for (int i = threadIdx.x / kG; i < s.n; i += groups) propose_absorption<kG>(s.absorption, i, lane);
+        for (int i = threadIdx.x / kG; i < s.n; i += groups) {
+            if (proposes(s.absorption, i)) propose_absorption<kG>(s.absorption, i, lane);
+            else if (lane == 0) s.absorption.proposal[i] = -1;
+        }
         __syncthreads();
-        for (int c = threadIdx.x / kG; c < s.n; c += groups) accept_absorption<kG>(s.absorption, c, lane);
+        for (int c = threadIdx.x / kG; c < s.n; c += groups)
+            if (accepts(s.absorption, c)) accept_absorption<kG>(s.absorption, c, lane);
         __syncthreads();
     }
     scan_in_block<4>(s.n + 1, s.size_of, s.pack);
@@ -1030,10 +1059,11 @@ std::unique_ptr<tf_transfer> aggregate(tf_ctx *ctx, const Csr<double, int32_t> &
         for (int round = 0; absorb && round < 2; ++round) {
             with_row_lanes(g, [&](auto lanes) {
                 constexpr int kG = decltype(lanes)::value;
-                const unsigned grid = grid_for(static_cast<int64_t>(n) * kG);
-                propose_absorption_kernel<kG><<<grid, kBlock, 0, ctx->stream>>>(n, s.absorption);
+                const unsigned lanes_grid = grid_for(static_cast<int64_t>(n) * kG);
+                propose_absorption_kernel<kG>
+                    <<<kG == 32 ? lanes_grid : grid_for(n), kBlock, 0, ctx->stream>>>(n, s.absorption);
                 launched(ctx, "propose_absorption");
-                accept_absorption_kernel<kG><<<grid, kBlock, 0, ctx->stream>>>(n, s.absorption);
+                accept_absorption_kernel<kG><<<lanes_grid, kBlock, 0, ctx->stream>>>(n, s.absorption);
                 launched(ctx, "accept_absorption");
             });
         }
