@@ -47,3 +47,16 @@ def test_single_precision_vectors(ctx, hierarchy, monkeypatch):
         amg.setup(a)
         out.append(amg.apply(b))
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("hierarchy", ["f32", "f64"])
+def test_vectors_in_host_memory(ctx, hierarchy):
+    a = to_device(P.heat3d(11, seed=5))
+    b = torch.tensor(P.rhs_uniform(a.rows, 10))
+    amg = tf.Amg(tf.amg_options(hierarchy_type=hierarchy, jacobi_weight=2 / 3), ctx=ctx)
+    amg.setup(a)
+    want = amg.apply(b.cuda()).cpu()
+    host, x = b.pin_memory(), torch.zeros_like(b).pin_memory()
+    for rhs, out in ((host, x), (b.cuda(), x), (host, torch.zeros_like(b, device="cuda"))):
+        x.zero_()
+        assert torch.equal(amg.apply(rhs, out).cpu(), want)

@@ -555,14 +555,19 @@ class HierarchyImpl final : public Hierarchy {
         if (outer) jacobi_zero_convert(ctx, f.n, f.dinv.data(), rhs, f.rhs.data(), f.x(), w_);
         else convert(ctx, f.n, rhs, f.rhs.data());
         if (const S *in = run_cycle(ctx, outer)) {
+            // (memory of the host is written by the conversion, in whole lines)
+            const bool direct = on_device(x);
             if constexpr (std::is_same_v<S, T>) {
-                jacobi_sweep(ctx, f.csr(), f.dinv.data(), f.rhs.data(), in, x, w_, nullptr, nullptr,
+                jacobi_sweep(ctx, f.csr(), f.dinv.data(), f.rhs.data(), in, direct ? x : f.x(), w_, nullptr, nullptr,
                              static_cast<const S *>(nullptr));
-                return;
-            } else if constexpr (std::is_same_v<S, float>) {
-                jacobi_sweep_widened(ctx, f.csr(), f.dinv.data(), f.rhs.data(), in, x, w_);
-                return;
+                if (direct) return;
             } else {
+                if constexpr (std::is_same_v<S, float>) {
+                    if (direct) {
+                        jacobi_sweep_widened(ctx, f.csr(), f.dinv.data(), f.rhs.data(), in, x, w_);
+                        return;
+                    }
+                }
                 jacobi_sweep(ctx, f.csr(), f.dinv.data(), f.rhs.data(), in, f.x(), w_, nullptr, nullptr,
                              static_cast<const S *>(nullptr));
             }

@@ -101,6 +101,10 @@ void pool_context_closed(int device) noexcept;
 // capture).
 void wait_for_device() noexcept;
 
+// Whether p is memory of the current device itself (not host, managed or a
+// peer's memory).
+bool on_device(const void *p);
+
 // The stream on which this thread's DeviceBuffers are allocated from the
 // pool, null outside PoolScope.
 inline thread_local const std::shared_ptr<StreamLife> *pool_stream = nullptr;

@@ -60,17 +60,6 @@ void check_types(int value_type, int index_type) {
     require(index_type == TF_I32 || index_type == TF_I64, "index type must be TF_I32 or TF_I64");
 }
 
-// Memory that kernels on this device may read and write.
-bool on_device(const void *p) {
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    int device = 0;
-    return a.type == cudaMemoryTypeDevice && cudaGetDevice(&device) == cudaSuccess && a.device == device;
-}
-
 bool disjoint(const void *a, const void *b, size_t bytes) {
     const auto pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);
     return pa + bytes <= pb || pb + bytes <= pa;

@@ -101,6 +101,16 @@ void *pool_allocate(int device, cudaStream_t stream, size_t bytes) {
     return p;
 }
 
+bool on_device(const void *p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    int device = 0;
+    return a.type == cudaMemoryTypeDevice && cudaGetDevice(&device) == cudaSuccess && a.device == device;
+}
+
 void wait_for_device() noexcept {
     void *p = nullptr;
     if (cudaMalloc(&p, 256) == cudaSuccess) cudaFree(p);
