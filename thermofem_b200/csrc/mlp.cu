@@ -486,6 +486,8 @@ int tf_mlp_sgd(tf_mlp *m, double lr, double momentum) {
         launch_kernel(m->ctx, "mlp_sgd", sgd_kernel, 1, kMlpBlock, 0, m->params.data(), m->velocity.data(),
                       m->grad.data(), m->rows, static_cast<float>(lr), static_cast<float>(momentum), m->bf16.data());
         m->rows = 0;
+        // (a failed step is this call's failure, and the batch's arrays are the caller's again)
+        cuda_check(cudaStreamSynchronize(m->ctx->stream), "sgd");
     });
 }
 
