@@ -66,8 +66,25 @@ void pool_context_closed(int device) noexcept {
     pool_trim(device);
 }
 
+namespace {
+// Calls of this thread inside the scope leave every stream capture in
+// progress alone (giving memory back ends a capture otherwise, also the
+// caller's own one around a call that uses temporary arrays).
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode{cudaStreamCaptureModeRelaxed};
+    RelaxedCapture() { swap(); }
+    ~RelaxedCapture() { swap(); }
+    RelaxedCapture(const RelaxedCapture &) = delete;
+    RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+    void swap() {
+        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) cudaGetLastError();
+    }
+};
+}  // namespace
+
 void pool_trim(int device) noexcept {
     std::lock_guard<std::mutex> lock(pool_mutex());
+    const RelaxedCapture relaxed;
     try {
         DevicePool &p = pool_of(device);
         uint64_t used = 0, reserved = 0;
