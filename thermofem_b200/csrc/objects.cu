@@ -65,6 +65,12 @@ bool disjoint(const void *a, const void *b, size_t bytes) {
     return pa + bytes <= pb || pb + bytes <= pa;
 }
 
+// Both start at a multiple of the element's size (kernels dereference them;
+// copies take any address).
+bool element_aligned(const void *a, const void *b, size_t size) {
+    return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % size == 0;
+}
+
 // After a component's buffers were freed (in the order of the context's
 // stream): they are the pool's once the stream has drained.
 void released(tf_ctx *ctx) {
@@ -365,9 +371,11 @@ int tf_jacobi_apply(tf_jacobi *j, const void *rhs, void *x) {
         tf_ctx *ctx = j->ctx;
         const size_t bytes = static_cast<size_t>(j->n) * type_size(j->value_type);
         // Device vectors that do not overlap are read and written where they
-        // are; others (host memory, rhs aliasing x) go through the component's
-        // own: three copies of the vectors, 15 us at 885k rows in FP64.
-        const bool direct = on_device(rhs) && on_device(x) && disjoint(rhs, x, bytes);
+        // are; others (host memory, rhs aliasing x, vectors off their elements'
+        // boundary) go through the component's own: three copies of the
+        // vectors, 15 us at 885k rows in FP64.
+        const bool direct = element_aligned(rhs, x, type_size(j->value_type)) && on_device(rhs) && on_device(x) &&
+                            disjoint(rhs, x, bytes);
         auto run = [&](auto t, const auto &banded) {
             using T = decltype(t);
             Csr<T, int32_t> c{j->n, j->n, j->nnz, j->rp.data(), j->ci.data(), reinterpret_cast<const T *>(j->val.data())};
