@@ -93,7 +93,12 @@ struct StreamLife {
 // The device memory pool (pool.cu): allocation in stream order; free bytes
 // beyond a bound go back to the device at pool_trim().
 void *pool_allocate(int device, cudaStream_t stream, size_t bytes);
+// Frees a block whose context is gone.
+void pool_free(int device, void *p) noexcept;
 void pool_trim(int device) noexcept;
+// Ends the destruction of buffers freed on a context's stream (which may be
+// gone): once the stream has drained they are the pool's, and trimmed.
+void pool_released(const StreamLife &life) noexcept;
 void pool_context_opened(int device);
 void pool_context_closed(int device) noexcept;
 // Waits for all work queued on the current device, on whatever stream, as
@@ -159,9 +164,10 @@ class DeviceBuffer {
             if (now != device_) cudaSetDevice(device_);
             if (life_ && life_->open) {
                 cudaFreeAsync(ptr_, life_->stream);
+            } else if (life_) {
+                pool_free(device_, ptr_);
             } else {
                 cudaFree(ptr_);
-                if (life_) pool_trim(device_);
             }
             if (now != device_) cudaSetDevice(now);
         }

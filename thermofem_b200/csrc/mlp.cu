@@ -327,6 +327,7 @@ TF_MLP_INST(double, int64_t)
 
 struct tf_mlp {
     tf_ctx *ctx{nullptr};
+    std::shared_ptr<tfb::StreamLife> life;  // the model may be destroyed after its context
     float omega_min{0}, omega_max{0};
     tfb::DeviceBuffer<float> params, velocity;
     tfb::DeviceBuffer<uint16_t> bf16;
@@ -370,6 +371,7 @@ int tf_mlp_create(tf_ctx *ctx, uint64_t seed, double omega_min, double omega_max
         PoolScope pool(ctx);
         auto m = std::make_unique<tf_mlp>();
         m->ctx = ctx;
+        m->life = ctx->life;
         m->omega_min = static_cast<float>(omega_min);
         m->omega_max = static_cast<float>(omega_max);
         m->params.allocate(kP);
@@ -389,8 +391,10 @@ int tf_mlp_create(tf_ctx *ctx, uint64_t seed, double omega_min, double omega_max
 int tf_mlp_destroy(tf_mlp *m) {
     return guard([&] {
         if (!m) return;
-        DeviceScope scope(m->ctx->device);
+        const std::shared_ptr<StreamLife> life = m->life;
+        DeviceScope scope(life->device);
         delete m;
+        pool_released(*life);
     });
 }
 

@@ -11,8 +11,11 @@
 
 using namespace tfb;
 
+// Every component shares its context's StreamLife: it may be destroyed after
+// its context.
 struct tf_amg {
     tf_ctx *ctx;
+    std::shared_ptr<StreamLife> life;
     int value_type, index_type;
     AmgConfig cfg;
     std::unique_ptr<Hierarchy> owned;
@@ -21,6 +24,7 @@ struct tf_amg {
 
 struct tf_jacobi {
     tf_ctx *ctx;
+    std::shared_ptr<StreamLife> life;
     int value_type, index_type;
     int sweeps;
     double weight;
@@ -34,6 +38,7 @@ struct tf_jacobi {
 
 struct tf_solver {
     tf_ctx *ctx;
+    std::shared_ptr<StreamLife> life;
     int value_type, index_type;
     std::unique_ptr<Krylov> k;
     std::unique_ptr<tf_amg> view;        // borrowed view of the AMG preconditioner
@@ -41,6 +46,7 @@ struct tf_solver {
 
 struct tf_batch {
     tf_ctx *ctx{nullptr};
+    std::shared_ptr<StreamLife> life;
     std::vector<tf_solver *> solvers;
     std::vector<int64_t> generations;  // of the solvers when the graph was built
     cudaGraphExec_t exec{nullptr};
@@ -71,11 +77,15 @@ bool element_aligned(const void *a, const void *b, size_t size) {
     return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % size == 0;
 }
 
-// After a component's buffers were freed (in the order of the context's
-// stream): they are the pool's once the stream has drained.
-void released(tf_ctx *ctx) {
-    cudaStreamSynchronize(ctx->stream);
-    pool_trim(ctx->device);
+// Destroys a component.  Its buffers are freed in the order of the context's
+// stream while that is open, and are the pool's once the stream has drained.
+template <class C>
+void destroy(C *c) {
+    if (!c) return;
+    const std::shared_ptr<StreamLife> life = c->life;
+    DeviceScope scope(life->device);
+    delete c;
+    pool_released(*life);
 }
 
 void check_matrix_types(const tf_csr *a, int value_type, int index_type) {
@@ -120,18 +130,12 @@ int tf_amg_create(tf_ctx *ctx, int value_type, int index_type, const tf_amg_opti
         require(out && opt, "null argument");
         *out = nullptr;
         check_types(value_type, index_type);
-        *out = new tf_amg{ctx, value_type, index_type, AmgConfig(*opt), nullptr, nullptr};
+        *out = new tf_amg{ctx, ctx->life, value_type, index_type, AmgConfig(*opt), nullptr, nullptr};
     });
 }
 
 int tf_amg_destroy(tf_amg *m) {
-    return guard([&] {
-        if (!m) return;
-        tf_ctx *ctx = m->ctx;
-        DeviceScope scope(ctx->device);
-        delete m;
-        released(ctx);
-    });
+    return guard([&] { destroy(m); });
 }
 
 int tf_amg_setup(tf_amg *m, const tf_csr *a) {
@@ -288,6 +292,7 @@ int tf_jacobi_create(tf_ctx *ctx, int value_type, int index_type, int sweeps, do
         if (sweeps < 1 || !std::isfinite(w) || w <= 0 || w >= 2) fail(TF_ERR_INVALID, "Invalid Jacobi parameters");
         auto *j = new tf_jacobi();
         j->ctx = ctx;
+        j->life = ctx->life;
         j->value_type = value_type;
         j->index_type = index_type;
         j->sweeps = sweeps;
@@ -297,13 +302,7 @@ int tf_jacobi_create(tf_ctx *ctx, int value_type, int index_type, int sweeps, do
 }
 
 int tf_jacobi_destroy(tf_jacobi *j) {
-    return guard([&] {
-        if (!j) return;
-        tf_ctx *ctx = j->ctx;
-        DeviceScope scope(ctx->device);
-        delete j;
-        released(ctx);
-    });
+    return guard([&] { destroy(j); });
 }
 
 int tf_jacobi_setup(tf_jacobi *j, const tf_csr *a) {
@@ -414,6 +413,7 @@ int tf_solver_create(tf_ctx *ctx, int kind, int value_type, int index_type, cons
         check_types(value_type, index_type);
         auto s = std::make_unique<tf_solver>();
         s->ctx = ctx;
+        s->life = ctx->life;
         s->value_type = value_type;
         s->index_type = index_type;
         s->k = make_krylov(kind, value_type, index_type, *opt, precond, amg_opt);
@@ -422,13 +422,7 @@ int tf_solver_create(tf_ctx *ctx, int kind, int value_type, int index_type, cons
 }
 
 int tf_solver_destroy(tf_solver *s) {
-    return guard([&] {
-        if (!s) return;
-        tf_ctx *ctx = s->ctx;
-        DeviceScope scope(ctx->device);
-        delete s;
-        released(ctx);
-    });
+    return guard([&] { destroy(s); });
 }
 
 int tf_solver_setup(tf_solver *s, const tf_csr *a) {
@@ -460,7 +454,7 @@ tf_amg *tf_solver_amg(tf_solver *s) {
     if (!s->view) {
         tf_amg_options o;
         tf_amg_options_default(&o);
-        s->view.reset(new tf_amg{s->ctx, s->value_type, s->index_type, AmgConfig(o), nullptr, s->k->amg()});
+        s->view.reset(new tf_amg{s->ctx, s->life, s->value_type, s->index_type, AmgConfig(o), nullptr, s->k->amg()});
     }
     s->view->h = s->k->amg();
     return s->view.get();
@@ -500,6 +494,7 @@ int tf_batch_create(tf_ctx *ctx, int count, tf_solver *const *solvers, tf_batch 
         require(count >= 1 && solvers != nullptr, "a batch needs at least one solver");
         auto b = std::make_unique<tf_batch>();
         b->ctx = ctx;
+        b->life = ctx->life;
         for (int k = 0; k < count; ++k) {
             require(solvers[k] != nullptr && solvers[k]->ctx == ctx, "batched solvers must share the batch context");
             for (int j = 0; j < k; ++j) require(solvers[j] != solvers[k], "a solver appears twice in the batch");
@@ -513,11 +508,7 @@ int tf_batch_create(tf_ctx *ctx, int count, tf_solver *const *solvers, tf_batch 
 }
 
 int tf_batch_destroy(tf_batch *b) {
-    return guard([&] {
-        if (!b) return;
-        DeviceScope scope(b->ctx->device);
-        delete b;
-    });
+    return guard([&] { destroy(b); });
 }
 
 int tf_batch_apply(tf_batch *b, const void *const *rhs, void *const *x, tf_solve_result *results) {

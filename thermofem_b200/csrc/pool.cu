@@ -25,6 +25,7 @@ constexpr uint64_t kPoolKeep = uint64_t(4) << 30;
 
 struct DevicePool {
     cudaMemPool_t pool{nullptr};
+    cudaStream_t stream{nullptr};  // of frees whose context is gone
     int contexts{0};
 };
 
@@ -47,6 +48,20 @@ DevicePool &pool_of(int device) {  // pool_mutex() held
     return p;
 }
 
+// Calls of this thread inside the scope leave every stream capture in
+// progress alone (giving memory back ends a capture otherwise, also the
+// caller's own one around a call that uses temporary arrays).
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode{cudaStreamCaptureModeRelaxed};
+    RelaxedCapture() { swap(); }
+    ~RelaxedCapture() { swap(); }
+    RelaxedCapture(const RelaxedCapture &) = delete;
+    RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+    void swap() {
+        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) cudaGetLastError();
+    }
+};
+
 }  // namespace
 
 void pool_context_opened(int device) {
@@ -66,22 +81,6 @@ void pool_context_closed(int device) noexcept {
     pool_trim(device);
 }
 
-namespace {
-// Calls of this thread inside the scope leave every stream capture in
-// progress alone (giving memory back ends a capture otherwise, also the
-// caller's own one around a call that uses temporary arrays).
-struct RelaxedCapture {
-    cudaStreamCaptureMode mode{cudaStreamCaptureModeRelaxed};
-    RelaxedCapture() { swap(); }
-    ~RelaxedCapture() { swap(); }
-    RelaxedCapture(const RelaxedCapture &) = delete;
-    RelaxedCapture &operator=(const RelaxedCapture &) = delete;
-    void swap() {
-        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) cudaGetLastError();
-    }
-};
-}  // namespace
-
 void pool_trim(int device) noexcept {
     std::lock_guard<std::mutex> lock(pool_mutex());
     const RelaxedCapture relaxed;
@@ -97,6 +96,30 @@ void pool_trim(int device) noexcept {
         if (reserved > keep && cudaMemPoolTrimTo(p.pool, keep) != cudaSuccess) cudaGetLastError();
     } catch (...) {
     }
+}
+
+// (cudaFree would give the block back, but leave it counted as used: the bound
+// of pool_trim() would rise with every such block)
+void pool_free(int device, void *p) noexcept {
+    {
+        std::lock_guard<std::mutex> lock(pool_mutex());
+        const RelaxedCapture relaxed;
+        try {
+            DevicePool &d = pool_of(device);
+            if (!d.stream)
+                cuda_check(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking), "cudaStreamCreate");
+            cuda_check(cudaFreeAsync(p, d.stream), "cudaFreeAsync");
+            cuda_check(cudaStreamSynchronize(d.stream), "cudaFreeAsync");
+        } catch (...) {
+            cudaGetLastError();
+        }
+    }
+    pool_trim(device);
+}
+
+void pool_released(const StreamLife &life) noexcept {
+    if (life.open && cudaStreamSynchronize(life.stream) != cudaSuccess) cudaGetLastError();
+    pool_trim(life.device);
 }
 
 void *pool_allocate(int device, cudaStream_t stream, size_t bytes) {
