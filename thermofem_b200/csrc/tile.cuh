@@ -1307,14 +1307,24 @@ PipeShape pipe_shape(int64_t rows, int64_t nnz, int sm_count, const PipeConfig &
 // Number of partial sums a reducing launch writes: one per 256-row block.
 inline int partials(int64_t rows) { return static_cast<int>(rows > 0 ? (rows + kThreads - 1) / kThreads : 1); }
 
+// The copy an operator carries besides its CSR arrays.
+enum : int { kNoCopy, kSlicedCopy, kSortedCopy, kBandedCopy };
+template <class T, class I, class V>
+int copy_kind(const Csr<T, I, V> &a) {
+    if (!a.sp) return kNoCopy;
+    return a.bd ? kBandedCopy : (a.perm ? kSortedCopy : kSlicedCopy);
+}
+
 // Process-wide cache of tuned configurations, keyed by the operator's shape
-// and storage (value, row offset and column entry sizes).
+// and storage (value, row offset and column entry sizes, the copy it
+// carries: a caller's CSR arrays and a component's copy of the same operator
+// each have a shape of their own).
 struct TuneKey {
     int64_t rows, nnz;
-    int vsize, isize, csize, sm_count;
+    int vsize, isize, csize, copy, sm_count;
     bool operator<(const TuneKey &o) const {
-        return std::tie(rows, nnz, vsize, isize, csize, sm_count) <
-               std::tie(o.rows, o.nnz, o.vsize, o.isize, o.csize, o.sm_count);
+        return std::tie(rows, nnz, vsize, isize, csize, copy, sm_count) <
+               std::tie(o.rows, o.nnz, o.vsize, o.isize, o.csize, o.copy, o.sm_count);
     }
 };
 inline std::mutex &tune_mutex() {
@@ -1325,28 +1335,29 @@ inline std::map<TuneKey, PipeConfig> &tune_cache() {
     static std::map<TuneKey, PipeConfig> m;
     return m;
 }
-// (values of type V under vectors of type T: V's size, plus 100 when the
-// two differ, so FP32 values under FP64 vectors keep shapes of their own)
-template <class T, class I, class C, class V = T>
-TuneKey tune_key(int64_t rows, int64_t nnz, int sm_count) {
-    return TuneKey{rows, nnz, static_cast<int>(sizeof(V)) + (std::is_same_v<T, V> ? 0 : 100),
-                   static_cast<int>(sizeof(I)), static_cast<int>(sizeof(C)), sm_count};
+// C: the column stream of the operator's row tiles (with_columns).  (Values of
+// type V under vectors of type T: V's size, plus 100 when the two differ, so
+// FP32 values under FP64 vectors keep shapes of their own.)
+template <class C, class T, class I, class V>
+TuneKey tune_key(const Csr<T, I, V> &a, int sm_count) {
+    return TuneKey{a.rows, a.nnz, static_cast<int>(sizeof(V)) + (std::is_same_v<T, V> ? 0 : 100),
+                   static_cast<int>(sizeof(I)), static_cast<int>(sizeof(C)), copy_kind(a), sm_count};
 }
-template <class T, class I, class C, class V = T>
-PipeConfig tuned_config(int64_t rows, int64_t nnz, int sm_count) {
+template <class C, class T, class I, class V>
+PipeConfig tuned_config(const Csr<T, I, V> &a, int sm_count) {
     std::lock_guard<std::mutex> lock(tune_mutex());
-    auto it = tune_cache().find(tune_key<T, I, C, V>(rows, nnz, sm_count));
+    auto it = tune_cache().find(tune_key<C>(a, sm_count));
     return it == tune_cache().end() ? PipeConfig{} : it->second;
 }
-template <class T, class I, class C, class V = T>
-bool has_config(int64_t rows, int64_t nnz, int sm_count) {
+template <class C, class T, class I, class V>
+bool has_config(const Csr<T, I, V> &a, int sm_count) {
     std::lock_guard<std::mutex> lock(tune_mutex());
-    return tune_cache().count(tune_key<T, I, C, V>(rows, nnz, sm_count)) != 0;
+    return tune_cache().count(tune_key<C>(a, sm_count)) != 0;
 }
-template <class T, class I, class C, class V = T>
-void store_config(int64_t rows, int64_t nnz, int sm_count, const PipeConfig &cfg) {
+template <class C, class T, class I, class V>
+void store_config(const Csr<T, I, V> &a, int sm_count, const PipeConfig &cfg) {
     std::lock_guard<std::mutex> lock(tune_mutex());
-    tune_cache()[tune_key<T, I, C, V>(rows, nnz, sm_count)] = cfg;
+    tune_cache()[tune_key<C>(a, sm_count)] = cfg;
 }
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -1372,7 +1383,7 @@ void configure(tf_ctx *ctx, const Csr<T, I, V> &a, const PipeConfig &cfg) {
         using C = std::remove_cv_t<std::remove_pointer_t<decltype(cols)>>;
         const PipeShape p = pipe_shape<V, I, C>(a.rows, a.nnz, ctx->sm_count, cfg);
         require(p.smem <= 200 * 1024, "stage ring exceeds shared memory");
-        store_config<T, I, C, V>(a.rows, a.nnz, ctx->sm_count, cfg);
+        store_config<C>(a, ctx->sm_count, cfg);
     });
 }
 
@@ -1438,7 +1449,7 @@ bool rarely_runs(const E &, long) {
 template <class T, class I, class C, class XS, class Epi, class V>
 void launch_pipe(tf_ctx *ctx, const Csr<T, I, V> &a, const C *cols, const XS &xs, const Epi &epi, const char *name,
                  const PipeConfig *force) {
-    const PipeConfig cfg = force ? *force : tuned_config<T, I, C, V>(a.rows, a.nnz, ctx->sm_count);
+    const PipeConfig cfg = force ? *force : tuned_config<C>(a, ctx->sm_count);
     const PipeShape p = pipe_shape<V, I, C>(a.rows, a.nnz, ctx->sm_count, cfg);
     const int early = ctx->stable && !rarely_runs(epi, 0) ? 1 : 0;
     auto grid = [&](int resident) {
@@ -1521,8 +1532,7 @@ void launch_sliced(tf_ctx *ctx, const Csr<T, I, V> &a, const XS &xs, const Epi &
 // when the operator has them, else its indices).
 template <class T, class I, class V>
 PipeConfig copy_config(tf_ctx *ctx, const Csr<T, I, V> &a) {
-    return a.cd ? tuned_config<T, I, int16_t, V>(a.rows, a.nnz, ctx->sm_count)
-                : tuned_config<T, I, I, V>(a.rows, a.nnz, ctx->sm_count);
+    return a.cd ? tuned_config<int16_t>(a, ctx->sm_count) : tuned_config<I>(a, ctx->sm_count);
 }
 
 // Launches the sliced kernel when the operator carries a sliced copy and its
@@ -1815,7 +1825,7 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     check_faults(ctx);
-    store_config<T, I, C, V>(a.rows, a.nnz, ctx->sm_count, best);
+    store_config<C>(a, ctx->sm_count, best);
     if (best_ms) *best_ms = best_t;
     return best;
 }
@@ -1838,7 +1848,7 @@ template <class T, class I, class V>
 void take_rule(tf_ctx *ctx, const Csr<T, I, V> &a) {
     with_columns(a, [&](auto cols) {
         using C = std::remove_cv_t<std::remove_pointer_t<decltype(cols)>>;
-        store_config<T, I, C, V>(a.rows, a.nnz, ctx->sm_count, rule_config(a));
+        store_config<C>(a, ctx->sm_count, rule_config(a));
     });
 }
 
@@ -1847,7 +1857,7 @@ template <class T, class I, class V>
 bool tuned(tf_ctx *ctx, const Csr<T, I, V> &a) {
     return with_columns(a, [&](auto cols) {
         using C = std::remove_cv_t<std::remove_pointer_t<decltype(cols)>>;
-        return has_config<T, I, C, V>(a.rows, a.nnz, ctx->sm_count);
+        return has_config<C>(a, ctx->sm_count);
     });
 }
 
