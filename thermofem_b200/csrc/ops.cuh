@@ -105,6 +105,12 @@ void autotune_spmv(tf_ctx *ctx, const Csr<T, I> &a, const T *x, T *y, int *stage
 // (THERMOFEM_B200_SLICED_SHAPE forces the full timing, and with it that shape).
 template <class T, class I, class V = T>
 void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y);
+// The row-tile shape of an operator that is set up and streams a copy beside
+// 4-byte columns, timed and cached for a caller's own CSR arrays of it
+// (tf_spmv after a solver's setup, 192^3 heat: 113.9 -> 110.5 us in FP64,
+// 90.5 -> 76.6 us in FP32, for 24 launches of the first setup of that size).
+template <class T, class I>
+void tune_rows(tf_ctx *ctx, Csr<T, I> a, const T *x, T *y);
 // The storage the SpMV family streams for a under its cached shape: true
 // (sliced copy, *entries its padded entry count) or false (CSR, *entries = nnz).
 template <class T, class I, class V = T>

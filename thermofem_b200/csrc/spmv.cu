@@ -715,6 +715,19 @@ void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y) {
     else tile::autotune(ctx, a, x, y, nullptr, !forced);
 }
 
+template <class T, class I>
+void tune_rows(tf_ctx *ctx, Csr<T, I> a, const T *x, T *y) {
+    if (!a.sp || a.cd || a.rows < tile::kTimedRows || std::getenv("THERMOFEM_B200_SLICED_SHAPE")) return;
+    a.sp = nullptr;
+    a.sv = nullptr;
+    a.sc = nullptr;
+    a.bd = nullptr;
+    a.perm = nullptr;
+    if (!tile::tuned(ctx, a)) tile::autotune(ctx, a, x, y, nullptr, true);
+}
+template void tune_rows<float, int32_t>(tf_ctx *, Csr<float, int32_t>, const float *, float *);
+template void tune_rows<double, int32_t>(tf_ctx *, Csr<double, int32_t>, const double *, double *);
+
 template <class T, class I, class V>
 bool streams_sliced(tf_ctx *ctx, const Csr<T, I, V> &a, int64_t entries_if_sliced, int64_t *entries) {
     bool sliced = false;
