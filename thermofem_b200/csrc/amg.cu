@@ -376,9 +376,8 @@ class HierarchyImpl final : public Hierarchy {
         fill_zero(ctx, l.n, l.rhs.data());
         tune_spmv(ctx, l.csr(), static_cast<const S *>(l.rhs.data()), l.r.data());
     }
-    void tune_finest_rows(tf_ctx *ctx) override {
-        Level<S, V> &l = levels_.front();
-        if constexpr (std::is_same_v<S, V>) tune_rows(ctx, l.csr(), static_cast<const S *>(l.rhs.data()), l.r.data());
+    void leave_finest_row_shape(tf_ctx *ctx) const override {
+        if constexpr (std::is_same_v<S, V>) leave_row_shape(ctx, levels_.front().csr());
     }
     void finish_setup(tf_ctx *ctx, PhaseMarks &marks) {
         visits.assign(levels_.size(), 0);

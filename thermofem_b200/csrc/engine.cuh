@@ -45,9 +45,9 @@ class Hierarchy {
     virtual const void *apply_open(tf_ctx *ctx, const double *rhs) = 0;
     virtual const void *apply_open(tf_ctx *ctx, const float *rhs) = 0;
     virtual int storage_type() const = 0;
-    // tune_rows for the finest operator (of a component whose caller has it
-    // in the hierarchy's own type).
-    virtual void tune_finest_rows(tf_ctx *ctx) = 0;
+    // leave_row_shape for the finest operator (of a component whose caller
+    // has it in the hierarchy's own type).
+    virtual void leave_finest_row_shape(tf_ctx *ctx) const = 0;
     virtual int64_t rows() const = 0;
     virtual int level_count() const = 0;
     virtual tf_csr level_matrix(int d) const = 0;

@@ -709,7 +709,7 @@ class KrylovImpl final : public Krylov {
         tiles_ = tile::partials(n_);
         fill_zero(ctx, n_, x_.data());
         tune_spmv(ctx, csr(), static_cast<const T *>(x_.data()), q_.data());
-        if constexpr (std::is_same_v<I, int32_t>) tune_rows(ctx, csr(), static_cast<const T *>(x_.data()), q_.data());
+        if constexpr (std::is_same_v<I, int32_t>) leave_row_shape(ctx, csr());
         parts_ = parts_for(n_);
         part_.allocate(static_cast<size_t>(2 * std::max(tiles_, parts_)));
         partb_.allocate(static_cast<size_t>(std::max(tiles_, parts_)));

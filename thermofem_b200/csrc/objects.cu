@@ -148,7 +148,7 @@ int tf_amg_setup(tf_amg *m, const tf_csr *a) {
         auto native = to_native(m->ctx, *a);
         const int storage = m->cfg.o.hierarchy_type == -1 ? m->value_type : m->cfg.o.hierarchy_type;
         auto h = build_hierarchy(m->ctx, m->cfg, storage, *native);
-        if (storage == m->value_type && m->index_type == TF_I32) h->tune_finest_rows(m->ctx);
+        if (storage == m->value_type && m->index_type == TF_I32) h->leave_finest_row_shape(m->ctx);
         m->owned = std::move(h);
         m->h = m->owned.get();
     });
@@ -278,7 +278,7 @@ int tf_amg_load(tf_amg *m, const char *path) {
         // transactional, as setup: the previous hierarchy stays on failure
         PoolScope pool(m->ctx);
         auto h = restore_hierarchy(m->ctx, m->cfg, storage, in);
-        if (storage == m->value_type && m->index_type == TF_I32) h->tune_finest_rows(m->ctx);
+        if (storage == m->value_type && m->index_type == TF_I32) h->leave_finest_row_shape(m->ctx);
         m->owned = std::move(h);
         m->h = m->owned.get();
     });

@@ -105,12 +105,16 @@ void autotune_spmv(tf_ctx *ctx, const Csr<T, I> &a, const T *x, T *y, int *stage
 // (THERMOFEM_B200_SLICED_SHAPE forces the full timing, and with it that shape).
 template <class T, class I, class V = T>
 void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y);
-// The row-tile shape of an operator that is set up and streams a copy beside
-// 4-byte columns, timed and cached for a caller's own CSR arrays of it
-// (tf_spmv after a solver's setup, 192^3 heat: 113.9 -> 110.5 us in FP64,
-// 90.5 -> 76.6 us in FP32, for 24 launches of the first setup of that size).
-template <class T, class I>
-void tune_rows(tf_ctx *ctx, Csr<T, I> a, const T *x, T *y);
+// The row-tile shape that the setup of a large stencil operator leaves for a
+// caller's own CSR arrays of it (where the caller tuned none): two rows per
+// thread, three CTAs per SM.  From 6M rows in FP64 and 2M in FP32, where it was
+// the best or equal to it on every operator timed, against the default: 184^3
+// to 256^3 heat and convection-diffusion FP64 101.1 -> 99.1, 113.5 -> 110.6,
+// 180.6 -> 176.5, 272.9 -> 265.9 us, FP32 80.9 -> 68.9 to 218.6 -> 176.7 us,
+// 600x60x60 FP32 30.7 -> 28.5 us; but 500x300x20 FP64 50.7 -> 53.6 us and
+// slower by 10 to 30 % at 300,000 to 540,000 rows.
+template <class T>
+void leave_row_shape(tf_ctx *ctx, Csr<T, int32_t> a);
 // The storage the SpMV family streams for a under its cached shape: true
 // (sliced copy, *entries its padded entry count) or false (CSR, *entries = nnz).
 template <class T, class I, class V = T>

@@ -715,18 +715,16 @@ void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y) {
     else tile::autotune(ctx, a, x, y, nullptr, !forced);
 }
 
-template <class T, class I>
-void tune_rows(tf_ctx *ctx, Csr<T, I> a, const T *x, T *y) {
-    if (!a.sp || a.cd || a.rows < tile::kTimedRows || std::getenv("THERMOFEM_B200_SLICED_SHAPE")) return;
+template <class T>
+void leave_row_shape(tf_ctx *ctx, Csr<T, int32_t> a) {
+    if (!a.bd || a.cd || a.rows < (sizeof(T) == 4 ? 2000000 : 6000000)) return;
     a.sp = nullptr;
     a.sv = nullptr;
-    a.sc = nullptr;
     a.bd = nullptr;
-    a.perm = nullptr;
-    if (!tile::tuned(ctx, a)) tile::autotune(ctx, a, x, y, nullptr, true);
+    if (!tile::tuned(ctx, a)) tile::configure(ctx, a, tile::PipeConfig{2, 3, 100, 2});
 }
-template void tune_rows<float, int32_t>(tf_ctx *, Csr<float, int32_t>, const float *, float *);
-template void tune_rows<double, int32_t>(tf_ctx *, Csr<double, int32_t>, const double *, double *);
+template void leave_row_shape<float>(tf_ctx *, Csr<float, int32_t>);
+template void leave_row_shape<double>(tf_ctx *, Csr<double, int32_t>);
 
 template <class T, class I, class V>
 bool streams_sliced(tf_ctx *ctx, const Csr<T, I, V> &a, int64_t entries_if_sliced, int64_t *entries) {

@@ -1685,8 +1685,7 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
     if (quick) {
         best = PipeConfig{2, 3, 125, 1};
         // (an operator with a copy streams that)
-        if (!copied)
-            tiles = {{2, 3, 125, 1}, {2, 4, 100, 1}, {2, 4, 125, 1}, {3, 2, 125, 1}, {2, 2, 100, 2}, {2, 3, 100, 2}};
+        if (!copied) tiles = {{2, 3, 125, 1}, {2, 4, 100, 1}, {2, 4, 125, 1}, {3, 2, 125, 1}, {2, 3, 100, 2}};
     } else {
         for (int rpt : {1, 2})
             for (int stages : {2, 3})
