@@ -153,8 +153,13 @@ bool on_device(const void *p) {
 
 void wait_for_device() noexcept {
     void *p = nullptr;
-    if (cudaMalloc(&p, 256) == cudaSuccess) cudaFree(p);
-    else cudaGetLastError();
+    if (cudaMalloc(&p, 256) == cudaSuccess) {
+        cudaFree(p);
+        return;
+    }
+    // (a full device)
+    cudaGetLastError();
+    if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
 }
 
 }  // namespace tfb
