@@ -291,7 +291,7 @@ class HierarchyImpl final : public Hierarchy {
             }
             marks.mark(ctx, kPhColumns);
             if (copies && !(banded_enabled() && build_banded(ctx, l.values(), found.shapes, bands.data(), l.sl)) &&
-                l.cd.data()) {
+                l.cd.data() && !streams_rows<S, V>(l.n, l.nnz)) {
                 if (sorted_slices_enabled()) build_sliced(ctx, l.values(), l.sl, true);
                 else build_sliced(ctx, l.values(), found.shapes, slices.data(), l.sl);
             }
@@ -368,7 +368,8 @@ class HierarchyImpl final : public Hierarchy {
             l.cd.allocate(static_cast<size_t>(l.nnz));
             if (!delta_columns(ctx, l.n, l.rp.data(), l.ci.data(), l.cd.data())) l.cd.release();
         }
-        if (sliced_enabled() && !(banded_enabled() && build_banded(ctx, l.values(), l.sl)) && l.cd.data())
+        if (sliced_enabled() && !(banded_enabled() && build_banded(ctx, l.values(), l.sl)) && l.cd.data() &&
+            !streams_rows<S, V>(l.n, l.nnz))
             build_sliced(ctx, l.values(), l.sl, true);
     }
     // Launch shape of this level's row-tile kernels (cached by shape).

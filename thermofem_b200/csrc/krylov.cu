@@ -695,7 +695,8 @@ class KrylovImpl final : public Krylov {
         if constexpr (std::is_same_v<I, int32_t>) {
             // a banded copy where the operator's slices share their column
             // offsets (stencils), else the 2-byte-offset sliced copy
-            if (sliced_enabled() && !(banded_enabled() && build_banded(ctx, csr(), sl_)) && cd_.data())
+            if (sliced_enabled() && !(banded_enabled() && build_banded(ctx, csr(), sl_)) && cd_.data() &&
+                !streams_rows<T, T>(n_, nnz_))
                 build_sliced(ctx, csr(), sl_, false);
         }
         hier_.reset();

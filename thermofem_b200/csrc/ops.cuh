@@ -100,11 +100,15 @@ template <class T, class I>
 void autotune_spmv(tf_ctx *ctx, const Csr<T, I> &a, const T *x, T *y, int *stages, int *ctas_per_sm, int *cap_pct,
                    int *rows_per_thread, float *ms);
 // The launch shape of an operator that is set up: the one cached for its
-// shape and storage; else by rule (fewer than 262,144 rows) or by timing the
-// few shapes that win on larger ones, and cached
+// shape and storage; else by rule (fewer than 262,144 rows and 4M entries) or by
+// timing the few shapes that win on larger ones, and cached
 // (THERMOFEM_B200_SLICED_SHAPE forces the full timing, and with it that shape).
 template <class T, class I, class V = T>
 void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y);
+// Whether such an operator (vectors T, values V) streams its row tiles by rule
+// even with a sliced copy, which it then need not have.
+template <class T, class V>
+bool streams_rows(int64_t rows, int64_t nnz);
 // The row-tile shape that the setup of a large stencil operator leaves for a
 // caller's own CSR arrays of it (where the caller tuned none): two rows per
 // thread, three CTAs per SM.  From 6M rows in FP64 and 2M in FP32, where it was

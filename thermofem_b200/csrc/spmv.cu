@@ -711,9 +711,23 @@ void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y) {
     // (a forced shape is taken by the full tuner)
     const bool forced = std::getenv("THERMOFEM_B200_SLICED_SHAPE") != nullptr;
     if (!forced && tile::tuned(ctx, a)) return;
-    if (!forced && a.rows < tile::kTimedRows) tile::take_rule(ctx, a);
+    if (!forced && a.rows < tile::kTimedRows && a.nnz < tile::kTimedEntries) tile::take_rule(ctx, a);
     else tile::autotune(ctx, a, x, y, nullptr, !forced);
 }
+
+template <class T, class V>
+bool streams_rows(int64_t rows, int64_t nnz) {
+    if (rows >= tile::kTimedRows || nnz >= tile::kTimedEntries || std::getenv("THERMOFEM_B200_SLICED_SHAPE")) return false;
+    Csr<T, int32_t, V> a{rows, rows, nnz};
+    const int32_t some_sp = 0;
+    const int16_t some_cd = 0;
+    a.sp = &some_sp;
+    a.cd = &some_cd;
+    return tile::rule_config(a).sliced == 0;
+}
+template bool streams_rows<float, float>(int64_t, int64_t);
+template bool streams_rows<double, double>(int64_t, int64_t);
+template bool streams_rows<double, float>(int64_t, int64_t);
 
 template <class T>
 void leave_row_shape(tf_ctx *ctx, Csr<T, int32_t> a) {

@@ -706,8 +706,10 @@ __global__ void __launch_bounds__(kThreads) sliced_kernel(int64_t rows, const in
         T y[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) y[g] = h.c[g] != kColPad ? xr(h.c[g]) : T(0);
-        // operands of the epilogue that wait for others of its own
-        if constexpr (requires { epi.late(pre); }) epi.late(pre);
+        // operands of the epilogue that wait for others of its own, where the
+        // row is one batch (over a longer loop they only take its registers:
+        // F-cycles of a 200,003-row graph FP32 1,690 -> 1,630 us without)
+        if constexpr (G > 8 && requires { epi.late(pre); }) epi.late(pre);
         T acc = T(0);
 #pragma unroll
         for (int g = 0; g < G; ++g) acc += h.v[g] * y[g];
@@ -1212,8 +1214,9 @@ struct PipeConfig {
 // PipeConfig::prefetch of the direct kernel for small operators: whole slices
 // of up to kWideEntries slots are loaded ahead of the dependency wait and all
 // their gathers are in flight at once, where 8 at a time take as many round
-// trips to L2 as the row has eighths (SMALLLEVELS).  It needs 100-150
-// registers, so it is taken where one CTA per SM holds the operator.
+// trips to L2 as the row has eighths.  It needs 100-150
+// registers, so it is taken where two CTAs per SM hold the operator (at the limit
+// of rows, 256 CTAs on 148 SMs).
 constexpr int kWideSlices = 2, kWideEntries = 24;
 constexpr int64_t kWideRows = 65536;
 
@@ -1606,27 +1609,54 @@ inline bool tune_log() {
     return on;
 }
 
-// The shape a setup takes for operators of fewer than kTimedRows rows without
-// timing anything.  Over 488 tuned operators (levels of heat, convection-
-// diffusion, 2-D and unstructured problems, three hierarchy types) the tuner's
-// choices there come down to these: row tiles in two stages, three CTAs per
-// SM (1.02-1.05 of the best shape's time on average, at launches of 4-10 us
-// whose own timing scatters by as much); copies read directly, three CTAs;
-// FP32 values under FP64 vectors staged (sliced) or prefetched (banded).
-constexpr int64_t kTimedRows = 262144;
+// The shape a setup takes without timing anything, for operators of fewer than
+// kTimedRows rows and kTimedEntries entries.  It goes by the mean row length,
+// since what bounds such a launch does: short rows are one round of gathers,
+// long ones a chain of them on the few SMs that the rows reach.  Measured (us a
+// product, back to back) on every level of graph, heat, convection-diffusion
+// and 2-D hierarchies of 8,009 to 1.7M rows in the three hierarchy types, row
+// tiles in thirteen shapes and copies in nine, and by whole cycles where that
+// left a choice:
+//  - row tiles: the default for short rows (146,053 rows of 11, FP32: 6.3, three
+//    CTAs 6.9); three stages, two CTAs for long ones (17,868 rows of 60, FP32:
+//    13.4, default 17.8); two rows per thread where they are very long or one
+//    tile holds them (1,944 of 323, FP32 values: W-cycle of the hierarchy 12.9
+//    ms, 14.1 with one row; 337 of 229, FP32: 45.9 and 59.8);
+//  - sliced copies of short rows: the wide kernel under kWideRows rows (18,269
+//    rows of 11, FP32: 2.3, row tiles 3.9), the direct one above;
+//  - of long rows, eight slots at a time: FP64 (337 rows of 229: 25.1, wide 31.7,
+//    row tiles 82.7; from 8,192 rows only past 100 entries, a row tile streams
+//    its matrix before the wait: 10,732 of 59, F-cycle 1,349 us, copy 1,400),
+//    FP32 from 200 entries (1,293 of 253: 48.5, wide 53.6, row tiles 93.2; but
+//    3,651 of 161: W-cycle 5.95 ms, row tiles 5.68);
+//  - FP32 values under FP64 vectors: wide up to 15 entries a row (18,269 of 11:
+//    3.0, row tiles 4.0), staged up to 23 (11,879 of 16: 4.4, wide 5.5, row
+//    tiles 4.7), then row tiles (4,895 of 172: 51.7, wide 144, other copies 114);
+//  - banded copies read directly, three CTAs (prefetched under FP64 vectors).
+constexpr int64_t kTimedRows = 262144, kTimedEntries = 4000000;
+constexpr int64_t kLongRows = 40;  // entries a row
 template <class T, class I, class V>
 PipeConfig rule_config(const Csr<T, I, V> &a) {
-    PipeConfig c{2, 3, 125, 1};
     constexpr bool same = std::is_same_v<T, V>;
+    const int64_t mean = a.rows > 0 ? a.nnz / a.rows : 0;
+    const bool wide = a.rows < kWideRows;
+    PipeConfig c{};
+    if (mean >= kLongRows && (wide || mean >= 128))
+        c = mean >= 200 || (a.rows <= 512 && mean >= 80) ? PipeConfig{3, 1, 125, 2} : PipeConfig{3, 2, 125, 1};
     if (a.sp && a.bd) {
         c.sliced = 1;
         c.prefetch = same ? 0 : 1;
         c.sliced_ctas = 3;
-    } else if (a.sp && a.cd) {
-        const bool wide = a.rows < kWideRows;
-        c.sliced = same || wide ? 1 : 2;
-        c.prefetch = wide ? kWideSlices : 0;
-        c.sliced_ctas = same || wide ? 3 : 2;
+    } else if (a.sp && a.cd && same) {
+        const bool chain = sizeof(T) == 4 ? mean >= 200 : mean >= kLongRows && (mean >= 100 || a.rows < 8192);
+        c.sliced = mean < kLongRows || chain ? 1 : 0;
+        c.prefetch = wide && !chain ? kWideSlices : 0;
+        c.sliced_ctas = 3;
+    } else if (a.sp && a.cd && mean < 24) {
+        const bool one = wide && mean < 16;
+        c.sliced = one ? 1 : 2;
+        c.prefetch = one ? kWideSlices : 0;
+        c.sliced_ctas = one ? 3 : 2;
     }
     return c;
 }
@@ -1684,8 +1714,10 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
     const bool copied = std::is_same_v<I, int32_t> && a.sp && (a.bd || std::is_same_v<C, int16_t>);
     if (quick) {
         best = PipeConfig{2, 3, 125, 1};
-        // (an operator with a copy streams that)
-        if (!copied) tiles = {{2, 3, 125, 1}, {2, 4, 100, 1}, {2, 4, 125, 1}, {3, 2, 125, 1}, {2, 3, 100, 2}};
+        // (an operator of short rows with a copy streams that)
+        const bool long_rows = a.nnz >= kLongRows * a.rows;
+        if (!copied || long_rows)
+            tiles = {{2, 3, 125, 1}, {2, 4, 100, 1}, {2, 4, 125, 1}, {3, 2, 125, 1}, {2, 3, 100, 2}};
     } else {
         for (int rpt : {1, 2})
             for (int stages : {2, 3})
@@ -1843,16 +1875,13 @@ PipeConfig autotune(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y, float 
     });
 }
 
-// Caches the shape of rule_config for operators of a's shape and storage.
-// Not where that is the storage of a caller's CSR arrays (no copy, indices as
-// given), whose entry only a timed shape replaces; the default is as good or
-// better there (graphs of 2,000 to 200,000 rows: equal in FP64, 9.1 us against
-// 9.7 us of the rule's at 200,000 rows in FP32).
+// Caches the shape of rule_config for operators of a's shape and storage.  (Where
+// that is the storage of a caller's CSR arrays, tf_spmv takes it too: the default
+// it has without, but for long rows.)
 template <class T, class I, class V>
 void take_rule(tf_ctx *ctx, const Csr<T, I, V> &a) {
     with_columns(a, [&](auto cols) {
         using C = std::remove_cv_t<std::remove_pointer_t<decltype(cols)>>;
-        if (std::is_same_v<T, V> && std::is_same_v<C, I> && copy_kind(a) == kNoCopy) return;
         store_config<C>(a, ctx->sm_count, rule_config(a));
     });
 }
