@@ -161,24 +161,29 @@ __global__ void k_reset(KState *s, KState init) {
     *s = init;
 }
 
-// Re-arms the WHILE nodes of the solve graph.  many: another round of
+// Re-arms the WHILE nodes of the solve graph.  lead: one more of the first
+// kLead iterations, which show the solve's rate; many: another round of
 // `unroll` iterations, while at least that many are to be expected at the
 // solve's own rate so far (an iteration after the end of the solve changes
 // nothing, but costs its kernels); one: one more iteration, while the
 // recurrence is running and below the iteration limit.
-__global__ void k_set_continue(cudaGraphConditionalHandle many, cudaGraphConditionalHandle one, int unroll,
-                               const KState *s) {
+constexpr int kLead = 2;
+struct LoopHandles {
+    cudaGraphConditionalHandle lead, many, one;
+};
+__global__ void k_set_continue(LoopHandles h, int unroll, const KState *s) {
     pdl_enter();
     const bool on = s->running && s->it < s->max_it;
     if (unroll > 1) {
+        cudaGraphSetConditional(h.lead, on && s->it < kLead ? 1u : 0u);
         bool more = on && s->it + unroll <= s->max_it;
         if (more && s->it > 0 && s->res < s->res0 && s->tol > 0) {
             const float left = logf(static_cast<float>(s->res / s->tol)) * static_cast<float>(s->it);
             more = left >= static_cast<float>(unroll) * logf(static_cast<float>(s->res0 / s->res));
         }
-        cudaGraphSetConditional(many, more ? 1u : 0u);
+        cudaGraphSetConditional(h.many, more ? 1u : 0u);
     }
-    cudaGraphSetConditional(one, on ? 1u : 0u);
+    cudaGraphSetConditional(h.one, on ? 1u : 0u);
 }
 
 template <class T, int kAhead = 1, class Fin = tile::NoFinal>
@@ -880,19 +885,23 @@ class KrylovImpl final : public Krylov {
     // Adds the whole solve to graph g as one independent branch: (with
     // reset, a kernel that loads the initial state) prefix, the iterations,
     // suffix.  The iterations are a conditional WHILE node of one, which
-    // re-arms its condition from the device state; short ones come in a
-    // first node of kUnroll at a time, since a turn of a WHILE node takes
+    // re-arms its condition from the device state; short ones come in a node
+    // of kUnroll at a time before it, since a turn of a WHILE node takes
     // 5.6 us on B200 (a kernel of a programmatic chain 0.85 us): 128^2 FP64 PCG,
     // 16 launches an iteration, 2.97 -> 2.51 ms with eight positions in flight
-    // (walk), and 4 % less with the gated refresh once per round.  Not in batches, whose other systems fill the gap and whose
-    // graph would take 1.7 ms longer to build (12 systems), nor above
-    // kUnrollLaunches, where the turn is under 5 % of the iteration.  Throws
-    // when CUDA refuses a step; the caller ends any capture left open.
+    // (walk), 2.46 ms with the gated refresh once per round.  The first kLead
+    // iterations come one by one before that, so that a solve of a few (a time
+    // step from a good guess) does not run a round of five: 40^3 transient step
+    // of one PCG iteration 360 us without, 215 us.  Not in batches, whose other
+    // systems fill the gap and whose graph would take 1.7 ms longer to build (12
+    // systems), nor above kUnrollLaunches, where the turn is under 5 % of the
+    // iteration.  Throws when CUDA refuses a step; the caller ends any capture
+    // left open.
     static constexpr int kUnroll = 5, kUnrollLaunches = 32;
     void add_solve_nodes(tf_ctx *ctx, cudaGraph_t g, bool reset) {
         const int64_t before = ctx->launches;
-        cudaGraphConditionalHandle many{}, one;
-        cuda_check(cudaGraphConditionalHandleCreate(&one, g, 0, cudaGraphCondAssignDefault), "condition");
+        LoopHandles h{};
+        cuda_check(cudaGraphConditionalHandleCreate(&h.one, g, 0, cudaGraphCondAssignDefault), "condition");
         cudaGraph_t out = nullptr;
         int unroll = 1;
         bool deferred = false;
@@ -908,26 +917,28 @@ class KrylovImpl final : public Krylov {
                                                      cudaStreamCaptureModeThreadLocal),
                        "capture body");
             for (int k = 1; k <= iterations; ++k) enqueue_iteration(ctx, k == iterations || !deferred);
-            launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, many, one, unroll, state_.data());
+            launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, h, unroll, state_.data());
             cuda_check(cudaStreamEndCapture(ctx->stream, &out), "capture body end");
             return ctx->launches - b0;
         };
-        cudaGraphNode_t loop, rounds = nullptr;
-        per_iteration_ = add_loop(one, 1, &loop);
+        cudaGraphNode_t loop, lead = nullptr, rounds = nullptr;
+        per_iteration_ = add_loop(h.one, 1, &loop);
         if (!reset && per_iteration_ <= kUnrollLaunches) {
             // PCG with a refresh interval of whole rounds (50 by default): the
             // refresh once per round, the iterations before it never due one
             deferred = kind_ == TF_SOLVER_CG && opt_.residual_refresh_interval % kUnroll == 0;
             unroll = kUnroll;
-            cuda_check(cudaGraphConditionalHandleCreate(&many, g, 0, cudaGraphCondAssignDefault), "condition");
-            add_loop(many, unroll, &rounds);
+            for (auto *p : {&h.lead, &h.many})
+                cuda_check(cudaGraphConditionalHandleCreate(p, g, 0, cudaGraphCondAssignDefault), "condition");
+            add_loop(h.lead, 1, &lead);
+            add_loop(h.many, unroll, &rounds);
         }
         const int64_t p0 = ctx->launches;
         cuda_check(cudaStreamBeginCaptureToGraph(ctx->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
                    "capture prefix");
         if (reset) launch_kernel(ctx, "k_reset", k_reset, 1, 1, 0, state_.data(), initial_state());
         enqueue_prefix(ctx);
-        launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, many, one, unroll, state_.data());
+        launch_kernel(ctx, "set_continue", k_set_continue, 1, 1, 0, h, unroll, state_.data());
         cudaStreamCaptureStatus st;
         const cudaGraphNode_t *deps = nullptr;
         size_t ndeps = 0;
@@ -936,10 +947,13 @@ class KrylovImpl final : public Krylov {
         cuda_check(cudaStreamEndCapture(ctx->stream, &out), "capture prefix end");
         prefix_launches_ = ctx->launches - p0;
         for (cudaGraphNode_t from : last) {
-            cudaGraphNode_t to = rounds ? rounds : loop;
+            cudaGraphNode_t to = lead ? lead : loop;
             cuda_check(cudaGraphAddDependencies(g, &from, &to, 1), "loop order");
         }
-        if (rounds) cuda_check(cudaGraphAddDependencies(g, &rounds, &loop, 1), "loop order");
+        if (lead) {
+            cuda_check(cudaGraphAddDependencies(g, &lead, &rounds, 1), "loop order");
+            cuda_check(cudaGraphAddDependencies(g, &rounds, &loop, 1), "loop order");
+        }
         const int64_t s0 = ctx->launches;
         cuda_check(cudaStreamBeginCaptureToGraph(ctx->stream, g, &loop, nullptr, 1, cudaStreamCaptureModeThreadLocal),
                    "capture suffix");

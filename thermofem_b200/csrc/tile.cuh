@@ -1625,13 +1625,14 @@ inline bool tune_log() {
 //  - sliced copies of short rows: the wide kernel under kWideRows rows (18,269
 //    rows of 11, FP32: 2.3, row tiles 3.9), the direct one above;
 //  - of long rows, eight slots at a time: FP64 (337 rows of 229: 25.1, wide 31.7,
-//    row tiles 82.7; from 8,192 rows only past 100 entries, a row tile streams
-//    its matrix before the wait: 10,732 of 59, F-cycle 1,349 us, copy 1,400),
+//    row tiles 82.7; 20,000 of 57: 28.5, row tiles 39.4; where such a copy pads
+//    by more than half it is not built, slices_fit),
 //    FP32 from 200 entries (1,293 of 253: 48.5, wide 53.6, row tiles 93.2; but
 //    3,651 of 161: W-cycle 5.95 ms, row tiles 5.68);
 //  - FP32 values under FP64 vectors: wide up to 15 entries a row (18,269 of 11:
 //    3.0, row tiles 4.0), staged up to 23 (11,879 of 16: 4.4, wide 5.5, row
-//    tiles 4.7), then row tiles (4,895 of 172: 51.7, wide 144, other copies 114);
+//    tiles 4.7), then row tiles (4,895 of 172: 51.7, wide 144, other copies 114)
+//    up to 349 (1,409 of 618: 157, row tiles 380);
 //  - banded copies read directly, three CTAs (prefetched under FP64 vectors).
 constexpr int64_t kTimedRows = 262144, kTimedEntries = 4000000;
 constexpr int64_t kLongRows = 40;  // entries a row
@@ -1648,9 +1649,13 @@ PipeConfig rule_config(const Csr<T, I, V> &a) {
         c.prefetch = same ? 0 : 1;
         c.sliced_ctas = 3;
     } else if (a.sp && a.cd && same) {
-        const bool chain = sizeof(T) == 4 ? mean >= 200 : mean >= kLongRows && (mean >= 100 || a.rows < 8192);
+        const bool chain = mean >= (sizeof(T) == 4 ? 200 : kLongRows);
         c.sliced = mean < kLongRows || chain ? 1 : 0;
         c.prefetch = wide && !chain ? kWideSlices : 0;
+        c.sliced_ctas = 3;
+    } else if (a.sp && a.cd && mean >= 350) {
+        c.sliced = 1;
+        c.prefetch = 0;
         c.sliced_ctas = 3;
     } else if (a.sp && a.cd && mean < 24) {
         const bool one = wide && mean < 16;
