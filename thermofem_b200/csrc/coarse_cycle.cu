@@ -118,16 +118,28 @@ struct Part {
     unsigned mag;
 };
 
-// The CTAs of a cluster: values of other CTAs' rows through distributed
-// shared memory, the cluster barrier between steps.
+// The CTAs of a region: a cluster (values of other CTAs' rows through
+// distributed shared memory, the cluster barrier between steps) or one CTA
+// alone (plain shared-memory loads, __syncthreads).
+template <bool kOne>
 struct Group {
-    __device__ __forceinline__ int rank() const { return static_cast<int>(cg::this_cluster().block_rank()); }
-    __device__ __forceinline__ void sync() const { cg::this_cluster().sync(); }
+    __device__ __forceinline__ int rank() const {
+        if constexpr (kOne) return 0;
+        else return static_cast<int>(cg::this_cluster().block_rank());
+    }
+    __device__ __forceinline__ void sync() const {
+        if constexpr (kOne) __syncthreads();
+        else cg::this_cluster().sync();
+    }
     // Value of row `row` of the vector that sits at `local` in every CTA.
     template <class S>
     __device__ __forceinline__ S load(S *local, int row, Part p) const {
-        const unsigned owner = p.mag ? __umulhi(static_cast<unsigned>(row), p.mag) : static_cast<unsigned>(row);
-        return *cg::this_cluster().map_shared_rank(local + (row - static_cast<int>(owner) * p.R), owner);
+        if constexpr (kOne) {
+            return local[row];
+        } else {
+            const unsigned owner = p.mag ? __umulhi(static_cast<unsigned>(row), p.mag) : static_cast<unsigned>(row);
+            return *cg::this_cluster().map_shared_rank(local + (row - static_cast<int>(owner) * p.R), owner);
+        }
     }
 };
 
@@ -205,13 +217,13 @@ __device__ __forceinline__ void restrict_own(const G &cl, unsigned char *sm, con
     }
 }
 
-template <class S>
+template <class S, bool kOne>
 __global__ void __launch_bounds__(kTailThreads, 1)
     tail_kernel(const TailHeader<S> *ghdr, const TailStepDev *gsteps, const TailCopy *copies, int first, int count,
                 ProgramIO<S> io, int root_cur, int early, int *fault) {
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ uint64_t load_bar;
-    const Group cl;
+    const Group<kOne> cl;
     const int rank = cl.rank();
     const int tid = threadIdx.x, nt = blockDim.x;
     if (!early) pdl_wait();
@@ -760,6 +772,7 @@ bool TailRegion<S>::plan(tf_ctx *ctx, const std::vector<TailLevel<S>> &levels, c
                          const double *inv, int dense_n, S w, int max_steps) {
     dev_.reset();
     cluster_ = 0;
+    laid_out_ = false;
     if (levels.empty() || levels.size() > static_cast<size_t>(kTailMaxLevels)) return false;
     // row offsets and aggregate offsets, to size every CTA's share
     std::vector<std::vector<int32_t>> rps(levels.size()), offs(levels.size());
@@ -783,7 +796,7 @@ bool TailRegion<S>::plan(tf_ctx *ctx, const std::vector<TailLevel<S>> &levels, c
     int max_optin = 0;
     cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device),
                "shared memory limit");
-    cuda_check(cudaFuncSetAttribute(tail_kernel<S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+    cuda_check(cudaFuncSetAttribute(tail_kernel<S, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
                "cluster attribute");
     // one CTA when the region fits there (no cluster barrier, no remote
     // loads), with the root's matrix in global memory if need be; else the
@@ -791,7 +804,11 @@ bool TailRegion<S>::plan(tf_ctx *ctx, const std::vector<TailLevel<S>> &levels, c
     if (plan_one_cta(ctx, levels, parent, rps, offs, inv, dense_n, w, max_steps, static_cast<size_t>(max_optin) - 1024))
         return true;
     auto h = std::make_unique<TailHeader<S>>();
-    for (int C : {kTailMaxCluster, 8, 4, 2}) {
+    // (C = 1, one CTA row by row, where only the padding of the image does not
+    // fit: levels of short rows with a dense one among them, whose slice is as
+    // long as it; 19 levels of 197 to 143 rows, FP64: V-cycle 260 us, 725 us with
+    // 16 CTAs)
+    for (int C : {1, kTailMaxCluster, 8, 4, 2}) {
         std::memset(h.get(), 0, sizeof(TailHeader<S>));
         h->levels = static_cast<int>(levels.size());
         h->dense_n = dense_n;
@@ -911,22 +928,26 @@ bool TailRegion<S>::plan(tf_ctx *ctx, const std::vector<TailLevel<S>> &levels, c
         bool tx_ok = true;
         for (int k = 0; k < C; ++k) tx_ok = tx_ok && tx[static_cast<size_t>(k)] < (1u << 20);
         if (!tx_ok) continue;
-        allow_region_smem<tail_kernel<S>>(bytes);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(C));
-        cfg.blockDim = dim3(kTailThreads);
-        cfg.dynamicSmemBytes = bytes;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = static_cast<unsigned>(C);
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, tail_kernel<S>, &cfg) != cudaSuccess || clusters < 1) {
-            cudaGetLastError();
-            continue;
+        if (C == 1) {
+            allow_region_smem<tail_kernel<S, true>>(bytes);
+        } else {
+            allow_region_smem<tail_kernel<S, false>>(bytes);
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(static_cast<unsigned>(C));
+            cfg.blockDim = dim3(kTailThreads);
+            cfg.dynamicSmemBytes = bytes;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = static_cast<unsigned>(C);
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, tail_kernel<S, false>, &cfg) != cudaSuccess || clusters < 1) {
+                cudaGetLastError();
+                continue;
+            }
         }
         std::vector<TailCopy> flat;
         for (int k = 0; k < C; ++k) {
@@ -1142,6 +1163,7 @@ bool TailRegion<S>::plan_one_cta(tf_ctx *ctx, const std::vector<TailLevel<S>> &l
         dev->levels = std::move(lv);
         dev_ = std::move(dev);
         cluster_ = 1;
+        laid_out_ = true;
         smem_ = bytes;
         max_steps_ = max_steps;
         levels_ = levels;
@@ -1230,7 +1252,7 @@ bool TailRegion<S>::add_entry(const std::vector<CoarseStep<S>> &rec, size_t firs
 
 template <class S>
 void TailRegion<S>::upload(tf_ctx *ctx) {
-    if (cluster_ == 1) {
+    if (laid_out_) {
         // the different steps, and their order
         std::vector<RegionStep> table;
         std::vector<uint16_t> order;
@@ -1284,7 +1306,7 @@ void TailRegion<S>::upload(tf_ctx *ctx) {
 template <class S>
 void TailRegion<S>::launch(tf_ctx *ctx, int entry, const ProgramIO<S> &io, int root_cur) const {
     const auto [first, count] = entries_.at(static_cast<size_t>(entry));
-    if (cluster_ == 1) {
+    if (laid_out_) {
         // a cycle that starts from the zero guess reads no iterate of the root
         const int op0 = steps_.at(static_cast<size_t>(first)).op;
         const int reads_x = op0 == kTZero || op0 == kTJacobiZero || op0 == kTDense ? 0 : 1;
@@ -1309,11 +1331,13 @@ void TailRegion<S>::launch(tf_ctx *ctx, int entry, const ProgramIO<S> &io, int r
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = static_cast<unsigned>(cluster_);
-    attr[na].val.clusterDim.y = 1;
-    attr[na].val.clusterDim.z = 1;
-    ++na;
+    if (cluster_ > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = static_cast<unsigned>(cluster_);
+        attr[na].val.clusterDim.y = 1;
+        attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
     if (ctx->pdl) {
         attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[na].val.programmaticStreamSerializationAllowed = 1;
@@ -1321,8 +1345,10 @@ void TailRegion<S>::launch(tf_ctx *ctx, int entry, const ProgramIO<S> &io, int r
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    allow_region_smem<tail_kernel<S>>(smem_);
-    cuda_check(cudaLaunchKernelEx(&cfg, tail_kernel<S>, static_cast<const TailHeader<S> *>(dev_->header.data()),
+    if (cluster_ > 1) allow_region_smem<tail_kernel<S, false>>(smem_);
+    else allow_region_smem<tail_kernel<S, true>>(smem_);
+    auto kernel = cluster_ > 1 ? tail_kernel<S, false> : tail_kernel<S, true>;
+    cuda_check(cudaLaunchKernelEx(&cfg, kernel, static_cast<const TailHeader<S> *>(dev_->header.data()),
                                   static_cast<const TailStepDev *>(dev_->steps.data()),
                                   static_cast<const TailCopy *>(dev_->copies.data()), first, count, io, root_cur,
                                   ctx->stable ? 1 : 0, ctx->fault),

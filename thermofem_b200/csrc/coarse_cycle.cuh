@@ -123,6 +123,7 @@ class TailRegion {
     std::vector<std::pair<int, int>> entries_;
     std::unique_ptr<TailDevice<S>> dev_;
     int cluster_{0}, max_steps_{0};
+    bool laid_out_{false};  // one CTA over its own image (plan_one_cta)
     size_t smem_{0};
 };
 

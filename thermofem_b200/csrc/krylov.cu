@@ -167,7 +167,8 @@ __global__ void k_reset(KState *s, KState init) {
 // solve's own rate so far (an iteration after the end of the solve changes
 // nothing, but costs its kernels); one: one more iteration, while the
 // recurrence is running and below the iteration limit.
-constexpr int kLead = 2;
+// (A whole round, so that PCG's refresh interval ends where a round does.)
+constexpr int kLead = 5;
 struct LoopHandles {
     cudaGraphConditionalHandle lead, many, one;
 };
@@ -892,12 +893,13 @@ class KrylovImpl final : public Krylov {
     // (walk), 2.46 ms with the gated refresh once per round.  The first kLead
     // iterations come one by one before that, so that a solve of a few (a time
     // step from a good guess) does not run a round of five: 40^3 transient step
-    // of one PCG iteration 360 us without, 215 us.  Not in batches, whose other
+    // of one PCG iteration 360 us without, 188 us.  Not in batches, whose other
     // systems fill the gap and whose graph would take 1.7 ms longer to build (12
     // systems), nor above kUnrollLaunches, where the turn is under 5 % of the
     // iteration.  Throws when CUDA refuses a step; the caller ends any capture
     // left open.
     static constexpr int kUnroll = 5, kUnrollLaunches = 32;
+    static_assert(kLead % kUnroll == 0);
     void add_solve_nodes(tf_ctx *ctx, cudaGraph_t g, bool reset) {
         const int64_t before = ctx->launches;
         LoopHandles h{};
