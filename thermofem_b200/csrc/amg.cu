@@ -294,6 +294,7 @@ class HierarchyImpl final : public Hierarchy {
                 l.cd.data() && !streams_rows<S, V>(l.n, l.nnz)) {
                 if (sorted_slices_enabled()) build_sliced(ctx, l.values(), l.sl, true);
                 else build_sliced(ctx, l.values(), found.shapes, slices.data(), l.sl);
+                if (l.sl.sp.data() && !copy_pays<S, V>(l.n, l.nnz, l.sl.entries)) l.sl.release();
             }
             marks.mark(ctx, kPhTuning);
             tune_level(ctx, l);
@@ -369,8 +370,10 @@ class HierarchyImpl final : public Hierarchy {
             if (!delta_columns(ctx, l.n, l.rp.data(), l.ci.data(), l.cd.data())) l.cd.release();
         }
         if (sliced_enabled() && !(banded_enabled() && build_banded(ctx, l.values(), l.sl)) && l.cd.data() &&
-            !streams_rows<S, V>(l.n, l.nnz))
+            !streams_rows<S, V>(l.n, l.nnz)) {
             build_sliced(ctx, l.values(), l.sl, true);
+            if (l.sl.sp.data() && !copy_pays<S, V>(l.n, l.nnz, l.sl.entries)) l.sl.release();
+        }
     }
     // Launch shape of this level's row-tile kernels (cached by shape).
     void tune_level(tf_ctx *ctx, Level<S, V> &l) {

@@ -162,13 +162,15 @@ __global__ void k_reset(KState *s, KState init) {
 }
 
 // Re-arms the WHILE nodes of the solve graph.  lead: one more of the first
-// kLead iterations, which show the solve's rate; many: another round of
+// kLead iterations, where the residual is within kNear of the tolerance and the
+// solve may be over after any of them; many: another round of
 // `unroll` iterations, while at least that many are to be expected at the
 // solve's own rate so far (an iteration after the end of the solve changes
 // nothing, but costs its kernels); one: one more iteration, while the
 // recurrence is running and below the iteration limit.
 // (A whole round, so that PCG's refresh interval ends where a round does.)
 constexpr int kLead = 5;
+constexpr double kNear = 1e4;
 struct LoopHandles {
     cudaGraphConditionalHandle lead, many, one;
 };
@@ -176,7 +178,7 @@ __global__ void k_set_continue(LoopHandles h, int unroll, const KState *s) {
     pdl_enter();
     const bool on = s->running && s->it < s->max_it;
     if (unroll > 1) {
-        cudaGraphSetConditional(h.lead, on && s->it < kLead ? 1u : 0u);
+        cudaGraphSetConditional(h.lead, on && s->it < kLead && s->res0 <= kNear * s->tol ? 1u : 0u);
         bool more = on && s->it + unroll <= s->max_it;
         if (more && s->it > 0 && s->res < s->res0 && s->tol > 0) {
             const float left = logf(static_cast<float>(s->res / s->tol)) * static_cast<float>(s->it);
@@ -890,10 +892,11 @@ class KrylovImpl final : public Krylov {
     // of kUnroll at a time before it, since a turn of a WHILE node takes
     // 5.6 us on B200 (a kernel of a programmatic chain 0.85 us): 128^2 FP64 PCG,
     // 16 launches an iteration, 2.97 -> 2.51 ms with eight positions in flight
-    // (walk), 2.46 ms with the gated refresh once per round.  The first kLead
-    // iterations come one by one before that, so that a solve of a few (a time
-    // step from a good guess) does not run a round of five: 40^3 transient step
-    // of one PCG iteration 360 us without, 188 us.  Not in batches, whose other
+    // (walk), 2.46 ms with the gated refresh once per round.  Solves that
+    // start near their tolerance (a time step from a good guess) take the first
+    // kLead iterations one by one: 40^3 transient step of one PCG iteration 360
+    // us in a round of five, 181 us.  The others do not, five turns more are 1.3
+    // % of a 128^2 solve.  Not in batches, whose other
     // systems fill the gap and whose graph would take 1.7 ms longer to build (12
     // systems), nor above kUnrollLaunches, where the turn is under 5 % of the
     // iteration.  Throws when CUDA refuses a step; the caller ends any capture

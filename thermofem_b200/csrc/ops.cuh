@@ -109,6 +109,12 @@ void tune_spmv(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y);
 // even with a sliced copy, which it then need not have.
 template <class T, class V>
 bool streams_rows(int64_t rows, int64_t nnz);
+// Whether such an operator's sliced copy of that many entries is kept: of FP32
+// values under FP64 vectors in very long rows only where it pads by a quarter
+// at most (3,849 rows of 468, 40 %: V-cycle of the hierarchy 2.15 ms, without the
+// copy 1.87; 1,409 rows of 618, 16 %: product 157 us, row tiles 380).
+template <class T, class V>
+bool copy_pays(int64_t rows, int64_t nnz, int64_t entries);
 // The row-tile shape that the setup of a large stencil operator leaves for a
 // caller's own CSR arrays of it (where the caller tuned none): two rows per
 // thread, three CTAs per SM.  From 6M rows in FP64 and 2M in FP32, where it was

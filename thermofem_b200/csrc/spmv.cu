@@ -725,6 +725,14 @@ bool streams_rows(int64_t rows, int64_t nnz) {
     a.cd = &some_cd;
     return tile::rule_config(a).sliced == 0;
 }
+template <class T, class V>
+bool copy_pays(int64_t rows, int64_t nnz, int64_t entries) {
+    if (std::is_same_v<T, V> || rows >= tile::kTimedRows || nnz >= tile::kTimedEntries) return true;
+    return nnz / rows < 350 || entries <= nnz + nnz / 4;
+}
+template bool copy_pays<float, float>(int64_t, int64_t, int64_t);
+template bool copy_pays<double, double>(int64_t, int64_t, int64_t);
+template bool copy_pays<double, float>(int64_t, int64_t, int64_t);
 template bool streams_rows<float, float>(int64_t, int64_t);
 template bool streams_rows<double, double>(int64_t, int64_t);
 template bool streams_rows<double, float>(int64_t, int64_t);
