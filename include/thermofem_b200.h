@@ -333,7 +333,9 @@ int tf_amg_last_visits(const tf_amg *m, int64_t *visits, int capacity);
 int tf_amg_setup_phases(const tf_amg *m, double *ms, int capacity);
 int tf_amg_setup_phase_count(void);
 const char *tf_amg_setup_phase_name(int phase);
-/* Level operator and transfer of the hierarchy (read-only device views). */
+/* Level operator and transfer of the hierarchy (read-only device views, in
+ * memory of the library's pool: copies to any device, no CUDA IPC and no
+ * access from a peer GPU). */
 int tf_amg_level_matrix(const tf_amg *m, int level, tf_csr *out);
 /* y = A_level x with the level's operator as the cycle streams it (its
  * storage type and column stream); x, y device vectors of the hierarchy's

@@ -69,8 +69,8 @@ __device__ __forceinline__ void sum_partials(const double *part, int parts, doub
 // over [0, n), in their order, with the loads of kAhead of them in flight.
 // A reduction over fewer than kAheadRows rows has a fixed partition of at
 // most 512 CTAs whose threads take eight positions each: bound by eight round
-// trips to L2 when taken one after another, by one with all in flight
-// (AHEAD).  Longer vectors fill the GPU with the loads of more threads.
+// trips to L2 when taken one after another, by one with all in flight.
+// Longer vectors fill the GPU with the loads of more threads.
 constexpr int64_t kAheadRows = int64_t(1) << 20;
 template <int kAhead, class Load, class Use>
 __device__ __forceinline__ void walk(int64_t n, const Load &load, const Use &use) {

@@ -10,6 +10,8 @@
 // What the pool keeps is bounded: free memory stays with it while a setup
 // runs, and at the end of every setup and destroy call pool_trim() returns
 // what exceeds kPoolKeep (all of it once the device's last context is gone).
+// A cudaMalloc of this process that finds no memory gets what the pool holds
+// free (seen on a filled device), so only other processes miss it.
 #include <map>
 #include <mutex>
 

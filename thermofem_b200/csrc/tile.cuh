@@ -1868,9 +1868,10 @@ PipeConfig autotune_columns(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y
 }
 
 // Times the feasible rows per thread, ring depths, CTAs per SM and chunk
-// capacities on this operator (two warm-up and five timed launches each,
-// CUDA events on the context stream) and caches the fastest for every later
-// launch over an operator of the same shape and storage.  y is overwritten.
+// capacities on this operator (two warm-up and five timed launches each, quick
+// one and three of a few shapes; CUDA events on the context stream) and caches
+// the fastest for every later launch over an operator of the same shape and
+// storage.  y is overwritten.
 template <class T, class I, class V>
 PipeConfig autotune(tf_ctx *ctx, const Csr<T, I, V> &a, const T *x, T *y, float *best_ms, bool quick = false) {
     if (a.rows == 0 || !aligned16(a.rp) || (a.nnz && (!aligned16(a.ci) || !aligned16(a.val)))) return PipeConfig{};
